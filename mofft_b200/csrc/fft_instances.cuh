@@ -215,12 +215,25 @@ size_t generic_smem(int L, int lines, int cols) {
   return 4 * words * sizeof(T);
 }
 
+// Runtime-chain kernels (inst_runtime_f32.cu, inst_runtime_f64.cu):
+// cudaErrorNotSupported when a pass's chain does not fit them.
+cudaError_t rt_launch_f32(const mofft_pass_args *p, cudaStream_t s);
+cudaError_t rt_launch_f64(const mofft_pass_args *p, cudaStream_t s);
+cudaError_t rt_prepare_f32();
+cudaError_t rt_prepare_f64();
+
 template <typename T, bool WIDE, int BANK = 0>
 struct GenericInst {
   static const void *func() {
     return reinterpret_cast<const void *>(&generic_kernel<T, WIDE, BANK>);
   }
   static cudaError_t launch(const mofft_pass_args *p, cudaStream_t s) {
+    if constexpr (BANK == 0 && !WIDE) {
+      // the loop below keeps the chains with more butterflies per line than a
+      // CTA has threads (explicit chains of small radices)
+      const cudaError_t err = sizeof(T) == 4 ? rt_launch_f32(p, s) : rt_launch_f64(p, s);
+      if (err != cudaErrorNotSupported) return err;
+    }
     GenericArgs<T> a;
     a.in = static_cast<const cplx_t<T> *>(p->in);
     a.out = static_cast<cplx_t<T> *>(p->out);
@@ -329,6 +342,9 @@ struct GenericInst {
 
 // Each instance file defines one of these.
 const Entry *entries_generic(int *count);
+const Entry *entries_generic_lt(int *count);
+const Entry *entries_generic_eo(int *count);
+const Entry *entries_generic_vr(int *count);
 const Entry *entries_rows_f32(int *count);
 const Entry *entries_rows_f64(int *count);
 const Entry *entries_cols_f32(int *count);

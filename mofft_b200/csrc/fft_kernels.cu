@@ -13,7 +13,9 @@ namespace {
 const std::vector<Entry> &registry() {
   static const std::vector<Entry> all = [] {
     std::vector<Entry> v;
-    const Entry *(*lists[])(int *) = {entries_generic, entries_rows_f32,
+    const Entry *(*lists[])(int *) = {entries_generic, entries_generic_lt,
+                                      entries_generic_eo, entries_generic_vr,
+                                      entries_rows_f32,
                                       entries_rows_f64, entries_cols_f32,
                                       entries_cols_f64, entries_rows_mixed,
                                       entries_cols_mixed, entries_tensor64,
@@ -52,7 +54,9 @@ extern "C" int mofft_cuda_prepare_device(void) {
         e.func(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
   }
-  return 0;
+  cudaError_t err = rt_prepare_f32();
+  if (err == cudaSuccess) err = rt_prepare_f64();
+  return (int)err;
 }
 
 extern "C" size_t mofft_cuda_kernel_aux_bytes(int kernel) {

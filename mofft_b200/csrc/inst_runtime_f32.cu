@@ -1,0 +1,9 @@
+// Runtime-chain kernels, float.
+#include "inst_runtime.cuh"
+
+namespace mofft {
+cudaError_t rt_launch_f32(const mofft_pass_args *p, cudaStream_t s) {
+  return rt_launch<float>(p, s);
+}
+cudaError_t rt_prepare_f32() { return rt_prepare<float>(); }
+}  // namespace mofft

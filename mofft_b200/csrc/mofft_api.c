@@ -31,6 +31,7 @@
 #include <string.h>
 #include <time.h>
 
+#include "generated/codelet_costs.h"
 #include "mofft_internal.h"
 #include "mofft_host.h"
 
@@ -353,6 +354,17 @@ static int make_pass(int precision_bits, unsigned bank, const int *chain,
   }
   const int g = generic_kernel_index(precision_bits, bank, chain + begin, count);
   if (g < 0) return 0;
+  int rt_lines, rt_threads;
+  size_t rt_smem;
+  if (bank == 0 && mofft_cuda_kernel_get(g)->radices[0] <= 16 &&
+      mofft_cuda_runtime_tile(precision_bits, !single, (int)length, chain + begin, count,
+                              single ? 1 : total / length, &rt_lines, &rt_threads, &rt_smem)) {
+    out->kernel = g;
+    out->kind = MOFFT_KERNEL_GENERIC;
+    out->lines = rt_lines;
+    out->smem_bytes = rt_smem;
+    return 1;
+  }
   int lines = single ? generic_rows_lines(precision_bits, (int)length)
                      : generic_cols_lines(precision_bits, (int)length, total,
                                           ns_outer);
@@ -477,8 +489,77 @@ int mofft_auto_radices(long long length, int *out, int capacity) {
   return n == 1 ? count : -1;
 }
 
+/* Cost of a runtime-chain line DFT, in instructions per point: each stage's
+ * codelet, an exchange, a barrier and the stage twiddles per stage boundary
+ * (about 16), and the registers a tile holds per point (threads = the most
+ * butterflies of any stage, each with the largest radix's footprint), which
+ * bound the points an SM has in flight. */
+static double runtime_chain_cost(int precision_bits, int cols, long long length,
+                                 long long line_units, const int *chain, int count) {
+  int lines, threads;
+  size_t smem;
+  if (!mofft_cuda_runtime_tile(precision_bits, cols, (int)length, chain, count, line_units,
+                               &lines, &threads, &smem))
+    return 1e6 + count;
+  double cost = 16.0 * (count - 1);
+  int lo = 64, hi = 0;
+  for (int i = 0; i < count; ++i) {
+    for (int k = 0; k < MOFFT_CODELET_COST_COUNT; ++k)
+      if (k_mofft_codelet_costs[k].radix == chain[i])
+        cost += (double)k_mofft_codelet_costs[k].instr / chain[i];
+    if (chain[i] < lo) lo = chain[i];
+    if (chain[i] > hi) hi = chain[i];
+  }
+  return cost + (double)(16 + 3 * hi) / lo;
+}
+
+typedef struct {
+  int precision_bits, cols;
+  long long length, line_units;
+  int chain[8], best[8];
+  int best_count;
+  double best_cost;
+} chain_search;
+
+static void search_runtime_chain(chain_search *s, long long rest, int most, int count) {
+  if (rest == 1) {
+    const double cost = runtime_chain_cost(s->precision_bits, s->cols, s->length,
+                                           s->line_units, s->chain, count);
+    if (cost < s->best_cost) {
+      s->best_cost = cost;
+      s->best_count = count;
+      memcpy(s->best, s->chain, (size_t)count * sizeof(int));
+    }
+    return;
+  }
+  if (count >= 8) return;
+  for (int r = most; r >= 2; --r) {
+    if (rest % r) continue;
+    s->chain[count] = r;
+    search_runtime_chain(s, rest / r, r, count + 1);
+  }
+}
+
+/* Cheapest chain of radices 2..16, largest first, for the runtime-chain
+ * kernels (0 when the length has none that fits them). */
+static int runtime_chain(int precision_bits, int cols, long long length, long long line_units,
+                         int *out, int capacity) {
+  chain_search s;
+  memset(&s, 0, sizeof(s));
+  s.precision_bits = precision_bits;
+  s.cols = cols;
+  s.length = length;
+  s.line_units = line_units;
+  s.best_cost = 1e6;
+  search_runtime_chain(&s, length, 16, 0);
+  if (s.best_count <= 0 || s.best_count > capacity) return 0;
+  memcpy(out, s.best, (size_t)s.best_count * sizeof(int));
+  return s.best_count;
+}
+
 /* Preferred chain of a pass of length L: the first registered specialised
- * kernel of that kind and length, else the generic default chain. */
+ * kernel of that kind and length, else the cheapest runtime chain (bank 0),
+ * else the generic default chain. */
 static int preferred_chain(int precision_bits, unsigned bank, int kind,
                            long long length, long long total,
                            long long ns_outer, int *out, int capacity) {
@@ -495,6 +576,12 @@ static int preferred_chain(int precision_bits, unsigned bank, int kind,
       }
       memcpy(out, d->radices, (size_t)d->radix_count * sizeof(int));
       return d->radix_count;
+    }
+    if (length <= 16384) {
+      const int cols = kind == MOFFT_KERNEL_COLS;
+      const int count = runtime_chain(precision_bits, cols, length, cols ? total / length : 1,
+                                      out, capacity);
+      if (count > 0) return count;
     }
   }
   return mofft_auto_radices(length, out, capacity);

@@ -1,0 +1,354 @@
+// Runtime-chain kernels: one CTA tile of a line DFT whose radix chain is a
+// launch argument, for the 13-smooth lengths without a compiled instance.
+//
+// A tile is `lines` lines of L points (ROWS: whole transforms; COLS: adjacent
+// super-butterflies of a multi-pass transform).  A thread runs at most one
+// butterfly per stage: it gathers R values into registers, multiplies the
+// stage twiddles, runs the straight-line radix-R codelet and, once every
+// thread of the CTA has read, scatters into the same shared-memory tile.  So
+// a tile needs one copy of its points (the ping-pong form this replaces kept
+// four component arrays), and every value crosses shared memory as one
+// {re, im} pair.
+//
+// Addresses.  With Ns the product of the radices applied so far, stage
+// (R, Ns) scatters butterfly j to (j / Ns) Ns R + (j mod Ns) + k Ns and the
+// next stage gathers j' + r L/R'.  The exchange between them inserts `pad`
+// pairs behind each block of Ns R points.  Both sides stay linear in k and r
+// (a block never divides L/R' unevenly), so an access costs one add, and the
+// divisions by Ns and by the butterflies per line are multiplications by a
+// precomputed reciprocal.  The pad makes the block pitch congruent to Ns
+// modulo one 128-byte row of pairs, which spreads consecutive butterflies
+// over distinct banks for every radix (without it the first stage's stride R
+// conflicts gcd(R, 16) ways).
+//
+// Tile shape.  The chain decides the threads (the most butterflies of any
+// stage), the register class its largest radix: variants for radices up to
+// 8, 11 and 16 keep short codelets at the occupancy they can have.
+//
+// Bound by: issue slots and latency (0.71 instructions per scheduler and cycle
+// at n = 343 before the stages were peeled), HBM for the short lengths that
+// run direct.  Measured per 2^25 FP32 / 2^24 FP64 points (HBM floor 82 us),
+// this against the ping-pong kernel: FP32 n = 100 801 -> 98 us, 343 1397 ->
+// 117, 1000 1005 -> 122, 3375 976 -> 128, 10000 1441 -> 214, 50625 (two
+// passes) 1849 -> 262; FP64 100 476 -> 86, 3375 672 -> 135, 50625 1233 -> 224.
+// Rel-L2 errors against 64 bits are those of the chain's codelets plus one
+// product per twiddle: FP32 3375 1.30e-7 -> 1.36e-7, 248832 1.92e-7 ->
+// 1.84e-7; FP64 3375 4.1e-16 -> 4.2e-16.
+#pragma once
+
+#include "fft_device.cuh"
+
+namespace mofft {
+
+constexpr int kRtMaxStages = 16;
+
+struct RtStage {
+  int radix;
+  int ns;               // product of the earlier radices
+  int bf;               // butterflies per line, L / radix
+  int twoff;            // stage table offset in the pass's twiddle table
+  unsigned magic_bf;    // ceil(2^32 / bf), 0 for bf == 1
+  unsigned magic_ns;    // ceil(2^32 / ns), 0 for ns == 1
+  int gpad;             // gather: pad pairs per block of ns points
+  int gstep;            // gather: words between a butterfly's inputs
+  int sblk;             // scatter: words between blocks of ns * radix points
+};
+
+template <typename T>
+struct RtArgs {
+  const cplx_t<T>* in;
+  cplx_t<T>* out;
+  const cplx_t<T>* tw;
+  const cplx_t<T>* tw_hi;
+  const cplx_t<T>* tw_lo;
+  long long batch;
+  long long in_dist;
+  long long out_dist;
+  long long ns_outer;       // COLS: product of the earlier passes' lengths
+  int total_lines;          // COLS: lines of one transform, M / L
+  int split_shift;
+  int length;               // L
+  int lines;                // lines of a full tile (COLS: a power of two)
+  int line_shift;           // COLS: log2 lines
+  int pitch;                // ROWS: pairs per line; COLS: pairs per element row
+  int stage_count;
+  unsigned magic_len;       // ceil(2^32 / L)
+  T sign_in;
+  T sign_out;
+  RtStage st[kRtMaxStages];
+};
+
+// n / d for n d < 2^32 with m = ceil(2^32 / d); m == 0 stands for d == 1.
+__device__ __forceinline__ int rt_div(int n, unsigned m) {
+  return m ? (int)__umulhi((unsigned)n, m) : n;
+}
+
+// Stage twiddles v[r] *= w^r.  w^1 .. w^4, w^8 and w^12 come from the table,
+// every other power is one product of two of them (w^4q * w^k), so a radix-16
+// butterfly needs 6 loads instead of 15 and no power carries more than one
+// extra rounding (every power from the table: 2-6 % slower, the error 1-4 %
+// smaller).
+template <typename T, int R>
+__device__ __forceinline__ void rt_twiddle(T (&vr)[R], T (&vi)[R],
+                                           const cplx_t<T>* __restrict__ tw, int ns) {
+  T wr[R], wi[R];
+#pragma unroll
+  for (int r = 1; r < R; ++r) {
+    if (r <= 3 || r % 4 == 0) {
+      const cplx_t<T> w = __ldg(tw + (r - 1) * ns);
+      wr[r] = w.x;
+      wi[r] = w.y;
+    } else {
+      const int h = r / 4 * 4, l = r % 4;
+      wr[r] = wr[h] * wr[l] - wi[h] * wi[l];
+      wi[r] = wr[h] * wi[l] + wi[h] * wr[l];
+    }
+    cmul<T>(vr[r], vi[r], wr[r], wi[r]);
+  }
+}
+
+// Kernel forms.  Stages are peeled (first / middle / last) so that each body
+// computes only the addresses it uses.
+enum RtMode {
+  kRtRows = 0,      // whole transforms, first and last stage on global memory
+  kRtStaged = 1,    // whole transforms copied through the tile
+  kRtColsHead = 2,  // first pass of a multi-pass transform (Ns = 1)
+  kRtColsTail = 3   // later pass: super-stage twiddles, strided stores
+};
+
+// One stage's butterfly: gathers from the tile or (SRC == kGlobal) global
+// memory, scatters likewise.
+template <typename T>
+struct RtIo {
+  bool act;
+  int src, sstep, dst, dstep;     // tile addresses, in pairs
+  const cplx_t<T>* gsrc;
+  cplx_t<T>* gdst;
+  long long gsstep, gdstep;
+  const cplx_t<T>* tw;            // this butterfly's stage twiddles
+  int ns;
+  T sign;
+};
+
+template <typename T, int R, Where SRC, Where DST, bool TW, class Super>
+__device__ __forceinline__ void rt_stage(const RtIo<T>& io, cplx_t<T>* sp, const Super& super) {
+  T vr[R], vi[R];
+  if (io.act) {
+    if constexpr (SRC == kGlobal) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const cplx_t<T> v = ld_global<T>(io.gsrc + r * io.gsstep);
+        vr[r] = v.x;
+        vi[r] = v.y * io.sign;
+      }
+      super(vr, vi);
+    } else {
+      const cplx_t<T>* p = sp + io.src;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const cplx_t<T> v = p[r * io.sstep];
+        vr[r] = v.x;
+        vi[r] = v.y;
+      }
+    }
+    if constexpr (TW) rt_twiddle<T, R>(vr, vi, io.tw, io.ns);
+    Dft<R>::fwd(vr, vi);
+  } else {
+    // defined on every path: a register that is only written under `act` and
+    // read under it behind the barrier counts as live around the stage loop,
+    // for every radix at once (the radix-8 class spilled 350 bytes a thread)
+#pragma unroll
+    for (int r = 0; r < R; ++r) vr[r] = vi[r] = T(0);
+  }
+  if constexpr (SRC == kShared && DST == kShared) __syncthreads();
+  if (io.act) {
+    if constexpr (DST == kGlobal) {
+#pragma unroll
+      for (int k = 0; k < R; ++k)
+        st_global<T>(io.gdst + k * io.gdstep, vr[k], vi[k] * io.sign);
+    } else {
+      cplx_t<T>* p = sp + io.dst;
+#pragma unroll
+      for (int k = 0; k < R; ++k) st_global<T>(p + k * io.dstep, vr[k], vi[k]);
+    }
+  }
+  if constexpr (DST == kShared) __syncthreads();
+}
+
+struct RtNoSuper {
+  template <typename T, int R>
+  __device__ __forceinline__ void operator()(T (&)[R], T (&)[R]) const {}
+};
+
+// Super-stage twiddle of a later column pass (ColsLayout's table form).
+template <typename T>
+struct RtSuper {
+  ColsLayout<T, 1, 1, true> lay;
+  int j, bf;
+  template <int R>
+  __device__ __forceinline__ void operator()(T (&vr)[R], T (&vi)[R]) const {
+    lay.template super_twiddle<R>(j, bf, vr, vi);
+  }
+};
+
+template <typename T, int MAXR, Where SRC, Where DST, bool TW, class Super>
+__device__ __forceinline__ void rt_dispatch(int radix, const RtIo<T>& io, cplx_t<T>* sp,
+                                            const Super& super) {
+#define MOFFT_RT_CASE(RR)                                                        \
+  case RR:                                                                       \
+    if constexpr (RR <= MAXR) rt_stage<T, RR, SRC, DST, TW>(io, sp, super);      \
+    break;
+  switch (radix) {
+    MOFFT_RT_CASE(2) MOFFT_RT_CASE(3) MOFFT_RT_CASE(4) MOFFT_RT_CASE(5)
+    MOFFT_RT_CASE(6) MOFFT_RT_CASE(7) MOFFT_RT_CASE(8) MOFFT_RT_CASE(9)
+    MOFFT_RT_CASE(10) MOFFT_RT_CASE(11) MOFFT_RT_CASE(12) MOFFT_RT_CASE(13)
+    MOFFT_RT_CASE(14) MOFFT_RT_CASE(15) MOFFT_RT_CASE(16)
+    default: break;
+  }
+#undef MOFFT_RT_CASE
+}
+
+template <typename T, int MODE, int MAXR, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1) rt_kernel(const __grid_constant__ RtArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx_t<T>* sp = reinterpret_cast<cplx_t<T>*>(smem_raw);
+  constexpr bool COLS = MODE >= kRtColsHead;
+  const int tid = threadIdx.x;
+  const int L = a.length;
+  const int last = a.stage_count - 1;
+  long long b;
+  int j0 = 0, nl;
+  if (COLS) {
+    const unsigned groups = (unsigned)(a.total_lines + a.lines - 1) >> a.line_shift;
+    const unsigned q = blockIdx.x / groups;
+    b = q;
+    j0 = (int)((blockIdx.x - q * groups) << a.line_shift);
+    nl = min(a.total_lines - j0, a.lines);
+  } else {
+    b = (long long)blockIdx.x * a.lines;
+    nl = (int)(a.batch - b < a.lines ? a.batch - b : a.lines);
+  }
+  const int step = COLS ? a.pitch : 1;   // pairs between a line's points
+  // this thread's butterfly j of line `line` in a stage of bf butterflies
+  auto place = [&](const RtStage& s, int& line, int& j) {
+    if (COLS) {
+      line = tid & (a.lines - 1);
+      j = tid >> a.line_shift;
+      return j < s.bf && line < nl;
+    }
+    line = rt_div(tid, s.magic_bf);
+    j = tid - line * s.bf;
+    return line < nl;
+  };
+  auto middle = [&](const RtStage& s) {
+    RtIo<T> io;
+    int line, j;
+    io.act = place(s, line, j);
+    const int base = COLS ? line : line * a.pitch;
+    const int jq = rt_div(j, s.magic_ns), jm = j - jq * s.ns;
+    io.src = base + (j + jq * s.gpad) * step;
+    io.sstep = s.gstep * step;
+    io.dst = base + (jq * s.sblk + jm) * step;
+    io.dstep = s.ns * step;
+    io.tw = a.tw + s.twoff + jm;
+    io.ns = s.ns;
+    rt_dispatch<T, MAXR, kShared, kShared, true>(s.radix, io, sp, RtNoSuper());
+  };
+
+  // ---- first stage: Ns = 1
+  {
+    const RtStage& s = a.st[0];
+    RtIo<T> io;
+    int line, j;
+    io.act = place(s, line, j);
+    const int base = COLS ? line : line * a.pitch;
+    io.dst = base + j * s.sblk * step;
+    io.dstep = step;
+    io.sign = a.sign_in;
+    if constexpr (MODE == kRtStaged) {
+      // the tile's lines as they lie in global memory, kBatch loads in flight
+      constexpr int kBatch = sizeof(T) == 4 ? 8 : 4;
+      const int points = nl * L;
+      const cplx_t<T>* src = a.in + b * a.in_dist;
+      for (int q0 = tid; q0 < points; q0 += kBatch * blockDim.x) {
+        cplx_t<T> v[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          const int q = q0 + k * (int)blockDim.x;
+          const int ln = (int)__umulhi((unsigned)q, a.magic_len);
+          if (q < points) v[k] = ld_global<T>(src + ln * a.in_dist + (q - ln * L));
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          const int q = q0 + k * (int)blockDim.x;
+          const int ln = (int)__umulhi((unsigned)q, a.magic_len);
+          if (q < points) {
+            v[k].y *= a.sign_in;
+            sp[ln * a.pitch + (q - ln * L)] = v[k];
+          }
+        }
+      }
+      __syncthreads();
+      io.src = base + j;
+      io.sstep = s.bf;
+      rt_dispatch<T, MAXR, kShared, kShared, false>(s.radix, io, sp, RtNoSuper());
+    } else if constexpr (MODE == kRtRows) {
+      io.gsrc = a.in + (b + line) * a.in_dist + j;
+      io.gsstep = s.bf;
+      rt_dispatch<T, MAXR, kGlobal, kShared, false>(s.radix, io, sp, RtNoSuper());
+    } else {
+      io.gsrc = a.in + b * a.in_dist + j0 + line + (long long)j * a.total_lines;
+      io.gsstep = (long long)a.total_lines * s.bf;
+      if constexpr (MODE == kRtColsHead) {
+        rt_dispatch<T, MAXR, kGlobal, kShared, false>(s.radix, io, sp, RtNoSuper());
+      } else {
+        RtSuper<T> super;
+        super.lay.tw_hi = a.tw_hi;
+        super.lay.tw_lo = a.tw_lo;
+        super.lay.split_shift = a.split_shift;
+        super.lay.jmod = (unsigned)(j0 + line) % (unsigned)a.ns_outer;
+        super.j = j;
+        super.bf = s.bf;
+        rt_dispatch<T, MAXR, kGlobal, kShared, false>(s.radix, io, sp, super);
+      }
+    }
+  }
+  constexpr bool kStores = MODE == kRtRows || MODE == kRtColsTail;
+  const int middles = kStores ? last : last + 1;
+  for (int i = 1; i < middles; ++i) middle(a.st[i]);
+  if constexpr (kStores) {
+    // ---- last stage: Ns R = L, so j mod Ns = j
+    const RtStage& s = a.st[last];
+    RtIo<T> io;
+    int line, j;
+    io.act = place(s, line, j);
+    const int base = COLS ? line : line * a.pitch;
+    io.src = base + j * step;
+    io.sstep = s.gstep * step;
+    io.tw = a.tw + s.twoff + j;
+    io.ns = s.ns;
+    io.sign = a.sign_out;
+    if constexpr (MODE == kRtRows) {
+      io.gdst = a.out + (b + line) * a.out_dist + j;
+      io.gdstep = s.ns;
+    } else {
+      const unsigned ns = (unsigned)a.ns_outer, jl = (unsigned)(j0 + line), q = jl / ns;
+      io.gdst = a.out + b * a.out_dist + (long long)q * ns * L + (jl - q * ns) + j * a.ns_outer;
+      io.gdstep = a.ns_outer * s.ns;
+    }
+    rt_dispatch<T, MAXR, kShared, kGlobal, true>(s.radix, io, sp, RtNoSuper());
+  } else {
+    // kRtColsHead: lines j0 .. j0+nl-1 are one contiguous block of the
+    // output; kRtStaged: the tile's lines leave as they arrived
+    const int points = nl * L;
+    cplx_t<T>* dst = COLS ? a.out + b * a.out_dist + (long long)j0 * L : a.out + b * a.out_dist;
+    for (int q = tid; q < points; q += blockDim.x) {
+      const int ln = (int)__umulhi((unsigned)q, a.magic_len);
+      const int i = q - ln * L;
+      const cplx_t<T> v = COLS ? sp[i * a.pitch + ln] : sp[ln * a.pitch + i];
+      st_global<T>(COLS ? dst + q : dst + ln * a.out_dist + i, v.x, v.y * a.sign_out);
+    }
+  }
+}
+
+}  // namespace mofft

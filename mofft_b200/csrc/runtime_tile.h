@@ -1,0 +1,39 @@
+// Tile shapes of the runtime-chain kernels (runtime_fft.cuh): one rule, used
+// by the planner (feasibility, reported lines and shared memory) and by the
+// launch (which also knows the batch).
+#pragma once
+
+#include <stddef.h>
+
+namespace mofft {
+
+// Most threads of a CTA: the launch bounds of the register class that runs a
+// chain's largest radix.  The register file divided by them is at or above
+// what the class needs unspilled (-Xptxas -v: FP32 37 / 48 / 63 registers for
+// radices up to 8 / 11 / 16, up to 80 in column passes with super-stage
+// twiddles; FP64 64 / 80 / 106, column passes 84 / 110 / 124).
+constexpr int rt_max_threads(int precision_bits, bool cols, int max_radix) {
+  if (precision_bits == 32) return max_radix <= 11 || !cols ? 1024 : 768;
+  if (max_radix <= 8) return cols ? 640 : 1024;
+  if (max_radix <= 11) return cols ? 512 : 768;
+  return 512;
+}
+
+struct RtShape {
+  int lines;       // lines per CTA
+  int threads;     // CTA threads: the most butterflies of any stage, whole warps
+  int max_radix;   // largest radix of the chain
+  int pitch;       // pairs per line (ROWS) / per element row (COLS)
+  int staged;      // ROWS: global I/O goes through the tile
+  int pad[16];     // pad pairs behind each block of the exchange after stage i
+  size_t smem;
+};
+
+// Shape of the tile of `length` points with stage list `chain` (first stage
+// first).  `units`: transforms of the launch (ROWS) or super-butterflies over
+// all of them (COLS); `line_units`: super-butterflies of one transform (COLS).
+// False when the chain does not fit the kernels.
+bool rt_shape(int precision_bits, bool cols, int length, const int *chain, int count,
+              long long units, long long line_units, RtShape *out);
+
+}  // namespace mofft

@@ -1,0 +1,69 @@
+"""Runtime-chain kernels (lengths without a compiled instance): every tile form
+at the sizes where it can go wrong, against the long-double oracle with the
+suite's bounds (5e-7 log2 n FP32, 2e-15 log2 n FP64)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import mofft_b200 as m
+import oracle
+from tests.conftest import cuda_available, fp32_tol, fp64_tol, rel_l2
+
+pytestmark = [pytest.mark.gpu,
+              pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")]
+
+CTYPE = {32: np.complex64, 64: np.complex128}
+
+# (length, explicit chain or None, batch).  Staged tiles (one stage, short
+# runs), direct rows of every register class, the thread limits, uneven radix
+# orders, column passes whose last tile is partial, three passes.
+CASES = [
+    (14, None, 1), (21, None, 600), (28, [2, 14], 257), (39, [13, 3], 33), (63, None, 4),
+    (77, None, 1001), (98, [7, 2, 7], 5), (108, None, 149), (143, None, 7), (210, None, 19),
+    (343, None, 3), (450, [2, 15, 3, 5], 9), (1001, None, 2), (1536, [2, 16, 6, 8], 3),
+    (2197, None, 5), (2744, [14, 14, 14], 2), (4095, None, 3), (5005, None, 2), (6561, None, 2),
+    (9009, None, 1), (12005, None, 1),
+    (4096, [2] * 12, 2),              # more butterflies than a CTA has threads
+    (28561, None, 3), (50625, None, 2), (30030, None, 1), (117649, None, 1), (531441, None, 1),
+]
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("n,chain,batch", CASES)
+def test_runtime_chain(n, chain, batch, bits):
+    import torch
+    dist = n + 3
+    buf = oracle.uniform(batch * dist, seed=n, dtype=CTYPE[bits])
+    lines = buf.reshape(batch, dist)[:, :n].astype(np.complex128)
+    x = torch.from_numpy(buf).cuda()
+    tol = fp32_tol(n) if bits == 32 else fp64_tol(n)
+    for direction in (m.FORWARD, m.BACKWARD):
+        ref = oracle.fft_ld(lines, direction)
+        for placement in (m.OUT_OF_PLACE, m.IN_PLACE):
+            y = x.clone() if placement == m.IN_PLACE else torch.zeros_like(x)
+            with m.Plan.create(n, direction, placement, bits=bits, batch=batch, distance=dist,
+                               radices=chain) as plan:
+                torch.cuda.synchronize()
+                plan.execute(y if placement == m.IN_PLACE else x, y)
+            out = y.cpu().numpy().reshape(batch, dist)
+            assert rel_l2(out[:, :n], ref) <= tol, (direction, placement)
+            gaps = buf.reshape(batch, dist)[:, n:] if placement == m.IN_PLACE else 0
+            assert np.all(out[:, n:] == gaps)          # nothing outside the lines
+
+
+def test_runtime_chain_dense_many_tiles():
+    """Dense batches with many full tiles and a partial last one."""
+    import torch
+    for bits in (32, 64):
+        for n, batch in ((20, 5000), (35, 4003), (100, 2001), (1000, 601), (3375, 301)):
+            x = oracle.uniform(n * batch, seed=batch, dtype=CTYPE[bits]).reshape(batch, n)
+            d = torch.from_numpy(x).cuda()
+            y = torch.empty_like(d)
+            with m.Plan.create(n, m.FORWARD, bits=bits, batch=batch) as plan:
+                plan.execute(d, y)
+            ref = oracle.fft_ld(x.astype(np.complex128), m.FORWARD)
+            got = y.cpu().numpy()
+            tol = fp32_tol(n) if bits == 32 else fp64_tol(n)
+            per = np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)
+            assert per.max() <= tol, (bits, n, int(np.argmax(per)))

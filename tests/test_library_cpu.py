@@ -444,3 +444,24 @@ def test_model_ranks_the_tuned_schedules():
     print(f"tuned schedule among the model's two best: {top2}/{total}")
     assert total >= 90 and top2 >= 0.6 * total
     assert m.model_seconds(4096, [byname["cols_float_64_t4_c32"]["index"]], 32, 1) == INF
+
+
+def test_every_smooth_length_has_a_schedule():
+    """Every 13-smooth length up to 2^14 and a spread above it: the planner's
+    chain multiplies to the length, its radices are the reference's, and the
+    tiles fit a CTA's shared memory."""
+    def smooth(n):
+        for p in (2, 3, 5, 7, 11, 13):
+            while n % p == 0:
+                n //= p
+        return n == 1
+
+    lengths = [n for n in range(2, 1 << 14) if smooth(n)]
+    lengths += [n for n in range(1 << 14, 1 << 20, 7) if smooth(n)][::9]
+    for bits in (32, 64):
+        for n in lengths:
+            s = m.schedule_preview(n, bits)
+            assert int(np.prod(s["radices"])) == n and int(np.prod(s["lengths"])) == n
+            assert s["pass_count"] <= 3
+            assert all(0 < b <= 227 * 1024 for b in s["smem_bytes"])
+            assert all(2 <= r <= 16 or r in (32, 64) for r in s["radices"])
