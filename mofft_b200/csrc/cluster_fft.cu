@@ -106,15 +106,16 @@ struct ClusterTileLayout {
   __device__ __forceinline__ int saddr(int i) const {
     return (i / CA) * (2 * BW) + c * (CA + 1) + (i % CA);
   }
-  __device__ __forceinline__ void gload(int, T& re, T& im) const {
-    re = T(0);
-    im = T(0);
+  template <int R, int NS>
+  __device__ __forceinline__ void gstore_run(int base, const T (&vr)[R], const T (&vi)[R]) const {
+    cplx_t<T>* p = gout + (long long)base * out_stride;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      if (active) st_global<T>(p, vr[k], vi[k] * sign);
+      p += (long long)NS * out_stride;
+    }
   }
-  __device__ __forceinline__ void gstore(int i, T re, T im) const {
-    if (active) st_global<T>(gout + (long long)i * out_stride, re, im * sign);
-  }
-  template <int R>
-  __device__ __forceinline__ void super_twiddle(int, int, T (&)[R], T (&)[R]) const {}
+  static constexpr bool kSuper = false;
 };
 
 constexpr int chain_table(const int* r, int n) {
@@ -251,12 +252,11 @@ struct ClusterBody<F, RadixList<HA...>, RadixList<RB...>> {
     for (int m = 0; m < PER; ++m) {
       const int j = ta + m * F::TPLA;
       if (EVEN || j < BF) {
+        if constexpr (sizeof...(HA) == 0) la.template gload_run<RL, BF>(j, vr[m], vi[m]);
 #pragma unroll
         for (int r = 0; r < RL; ++r) {
           const int idx = j + r * BF;
-          if constexpr (sizeof...(HA) == 0) {
-            la.gload(idx, vr[m][r], vi[m][r]);
-          } else {
+          if constexpr (sizeof...(HA) != 0) {
             vr[m][r] = la.sre[la.saddr(idx)];
             vi[m][r] = la.sim[la.saddr(idx)];
           }

@@ -138,8 +138,18 @@ struct RowsLayout {
   __device__ __forceinline__ void gstore(int i, T re, T im) const {
     if (active) st_global<T>(gout + i, re, im * sign);
   }
-  template <int R>
-  __device__ __forceinline__ void super_twiddle(int, int, T (&)[R], T (&)[R]) const {}
+  // v[r] = element j + r * BF; element base + k * NS = v[k]
+  template <int R, int BF>
+  __device__ __forceinline__ void gload_run(int j, T (&vr)[R], T (&vi)[R]) const {
+#pragma unroll
+    for (int r = 0; r < R; ++r) gload(j + r * BF, vr[r], vi[r]);
+  }
+  template <int R, int NS>
+  __device__ __forceinline__ void gstore_run(int base, const T (&vr)[R], const T (&vi)[R]) const {
+#pragma unroll
+    for (int k = 0; k < R; ++k) gstore(base + k * NS, vr[k], vi[k]);
+  }
+  static constexpr bool kSuper = false;
 };
 
 // A line whose shared-memory exchanges move {re, im} pairs: one 8-byte
@@ -195,72 +205,86 @@ struct ColsLayout {
   // super-stage twiddle on load: W^{e}, e = jmod * i, two-level table
   const cplx_t<T>* tw_hi;
   const cplx_t<T>* tw_lo;
-  long long jmod;         // (j mod Ns_outer) of this line
+  unsigned jmod;          // (j mod Ns_outer) of this line, below 2^32
+  cplx_t<T>* sw;          // the tile's R x C table of line powers (TW)
   int split_shift;        // K = 1 << split_shift
   __device__ __forceinline__ int saddr(int i) const { return i * PITCH + c; }
-  __device__ __forceinline__ void gload(int i, T& re, T& im) const {
-    if (active) {
-      const cplx_t<T> v = ld_global<T>(gin + (long long)i * in_stride);
-      re = v.x;
-      im = v.y * sign_in;
-    } else {
-      re = T(0);
-      im = T(0);
+  // v[r] = element j + r * BF of this line: one pointer walks the strided
+  // elements (a 64-bit product per element otherwise)
+  template <int R, int BF>
+  __device__ __forceinline__ void gload_run(int j, T (&vr)[R], T (&vi)[R]) const {
+    const cplx_t<T>* p = gin + (long long)j * in_stride;
+    const long long step = (long long)BF * in_stride;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (active) {
+        const cplx_t<T> v = ld_global<T>(p);
+        vr[r] = v.x;
+        vi[r] = v.y * sign_in;
+      } else {
+        vr[r] = vi[r] = T(0);
+      }
+      p += step;
     }
   }
-  // W^e from the two-level table (entry 0 of both tables is exactly 1).
-  __device__ __forceinline__ void super_w(long long e, T& wr, T& wi) const {
-    const cplx_t<T> hi = __ldg(tw_hi + (e >> split_shift));
-    const cplx_t<T> lo = __ldg(tw_lo + (e & ((1LL << split_shift) - 1)));
+  // W^e, e = jmod * i, from the two-level table (entry 0 of both tables is
+  // exactly 1).  The product has up to 48 bits, its upper part (below 2^32)
+  // comes out of one funnel shift.
+  __device__ __forceinline__ void super_w(unsigned i, T& wr, T& wi) const {
+    const unsigned long long e = (unsigned long long)jmod * i;
+    const unsigned lo_bits = (unsigned)e;
+    const unsigned hi_index = __funnelshift_r(lo_bits, (unsigned)(e >> 32), split_shift);
+    const cplx_t<T> hi = __ldg(tw_hi + hi_index);
+    const cplx_t<T> lo = __ldg(tw_lo + (lo_bits & ((1u << split_shift) - 1u)));
     wr = hi.x;
     wi = hi.y;
     cmul<T>(wr, wi, lo.x, lo.y);
   }
-  // Super-stage twiddle of butterfly j's loaded inputs (TW: passes with
-  // Ns_outer > 1): v[r] *= W^{jmod (j + r BF)}, no branch, so that every
-  // load issues together.  For R <= 16 it is W^{jmod j} u^r with
-  // u = W^{jmod BF}: u, u^2, u^4, u^8 come from the table and every other
-  // power is a product of two earlier ones (at most three products in a
-  // chain), so a butterfly needs at most five lookups instead of R.
-  template <int R>
-  __device__ __forceinline__ void super_twiddle(int j, int BF, T (&vr)[R], T (&vi)[R]) const {
-    if constexpr (TW) {
-      if constexpr (R <= 16) {
-        T ur[R], ui[R];
-        T br, bi;
-        super_w(jmod * (long long)j, br, bi);
-        const long long u = jmod * (long long)BF;
-#pragma unroll
-        for (int k = 1; k < R; k <<= 1) super_w(u * k, ur[k], ui[k]);
-#pragma unroll
-        for (int r = 3; r < R; ++r) {
-          if ((r & (r - 1)) == 0) continue;          // a power of two: loaded
-          int h = 1;
-          while (h * 2 <= r) h *= 2;                 // highest power of two in r
-          const int l = r - h;
-          ur[r] = ur[h] * ur[l] - ui[h] * ui[l];
-          ui[r] = ur[h] * ui[l] + ui[h] * ur[l];
-        }
-        cmul<T>(vr[0], vi[0], br, bi);
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-          T xr = ur[r], xi = ui[r];
-          cmul<T>(xr, xi, br, bi);
-          cmul<T>(vr[r], vi[r], xr, xi);
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          T xr, xi;
-          super_w(jmod * (long long)(j + r * BF), xr, xi);
-          cmul<T>(vr[r], vi[r], xr, xi);
-        }
-      }
+  // Super-stage twiddle of a butterfly's loaded inputs (TW: passes with
+  // Ns_outer > 1): v[r] *= W^{jmod (j + r BF)} = b u^r with b = W^{jmod j},
+  // u = W^{jmod BF}.  The powers u^r depend on the line only, so the tile's C
+  // lines share a table of R x C of them, filled once per tile from the
+  // two-level table; a thread then looks up its own b and reads u^r from
+  // shared memory.  (Every thread looking up u .. u^3, u^4, u^8, u^12 for
+  // itself: 14 loads and the index arithmetic of seven table entries per
+  // butterfly, 13 instructions a point; the second pass of FP32 65536 took
+  // 109 us of 2^25 points where the first, without twiddles, took 85.)
+  template <int R, int BF, int THREADS>
+  __device__ __forceinline__ void super_fill() const {
+    ColsLayout l = *this;
+    for (int q = threadIdx.x; q < R * C; q += THREADS) {
+      l.jmod = jmod - (unsigned)c + (unsigned)(q % C);   // C divides Ns_outer
+      T wr, wi;
+      l.super_w((unsigned)(q / C * BF), wr, wi);
+      st_global<T>(sw + q, wr, wi);
     }
   }
-  __device__ __forceinline__ void gstore(int i, T re, T im) const {
-    if (active) st_global<T>(gout + (long long)i * out_stride, re, im * sign_out);
+  template <int R>
+  __device__ __forceinline__ void super_twiddle(int j, T (&vr)[R], T (&vi)[R]) const {
+    T br, bi;
+    super_w((unsigned)j, br, bi);
+    cmul<T>(vr[0], vi[0], br, bi);
+#pragma unroll
+    for (int r = 1; r < R; ++r) {
+      const cplx_t<T> u = sw[r * C + c];
+      T xr = u.x, xi = u.y;
+      cmul<T>(xr, xi, br, bi);
+      cmul<T>(vr[r], vi[r], xr, xi);
+    }
   }
+  // element base + k * NS = v[k]
+  template <int R, int NS>
+  __device__ __forceinline__ void gstore_run(int base, const T (&vr)[R], const T (&vi)[R]) const {
+    cplx_t<T>* p = gout + (long long)base * out_stride;
+    const long long step = (long long)NS * out_stride;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      if (active) st_global<T>(p, vr[k], vi[k] * sign_out);
+      p += step;
+    }
+  }
+  static constexpr bool kSuper = TW;
+  static constexpr int kLines = C;
 };
 
 // Kernel flags (template parameter FLAGS of the ROWS kernels).
@@ -345,25 +369,39 @@ __device__ __forceinline__ void reg_stage(const Layout& lay, int t,
   constexpr int BF = L / R;
   constexpr int PER = (BF + TPL - 1) / TPL;
   constexpr bool EVEN = (BF % TPL) == 0;
+  constexpr bool SUPER = SRC == kGlobal && Layout::kSuper;
   T vr[PER][R];
   T vi[PER][R];
+  if constexpr (SUPER) {
+    // all of the tile's loads are in flight while its table is filled
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+      const int j = t + m * TPL;
+      if (EVEN || j < BF) lay.template gload_run<R, BF>(j, vr[m], vi[m]);
+    }
+    lay.template super_fill<R, BF, TPL * Layout::kLines>();
+    __syncthreads();
+  }
 #pragma unroll
   for (int m = 0; m < PER; ++m) {
     const int j = t + m * TPL;
     if (EVEN || j < BF) {
+      if constexpr (SUPER) {
+        lay.template super_twiddle<R>(j, vr[m], vi[m]);
+      } else if constexpr (SRC == kGlobal) {
+        lay.template gload_run<R, BF>(j, vr[m], vi[m]);
+      } else {
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int idx = j + r * BF;
-        if (SRC == kGlobal) {
-          lay.gload(idx, vr[m][r], vi[m][r]);
-        } else if constexpr (IsPairLayout<Layout>::value) {
-          lay.sget(idx, vr[m][r], vi[m][r]);
-        } else {
-          vr[m][r] = lay.sre[lay.saddr(idx)];
-          vi[m][r] = lay.sim[lay.saddr(idx)];
+        for (int r = 0; r < R; ++r) {
+          const int idx = j + r * BF;
+          if constexpr (IsPairLayout<Layout>::value) {
+            lay.sget(idx, vr[m][r], vi[m][r]);
+          } else {
+            vr[m][r] = lay.sre[lay.saddr(idx)];
+            vi[m][r] = lay.sim[lay.saddr(idx)];
+          }
         }
       }
-      if constexpr (SRC == kGlobal) lay.template super_twiddle<R>(j, BF, vr[m], vi[m]);
       if (NS > 1) {
         const int jm = j % NS;
         if constexpr (DTW && R == 16) {
@@ -387,16 +425,18 @@ __device__ __forceinline__ void reg_stage(const Layout& lay, int t,
     const int j = t + m * TPL;
     if (EVEN || j < BF) {
       const int base = (j / NS) * NS * R + (j % NS);
+      if constexpr (DST == kGlobal) {
+        lay.template gstore_run<R, NS>(base, vr[m], vi[m]);
+      } else {
 #pragma unroll
-      for (int k = 0; k < R; ++k) {
-        const int idx = base + k * NS;
-        if (DST == kGlobal) {
-          lay.gstore(idx, vr[m][k], vi[m][k]);
-        } else if constexpr (IsPairLayout<Layout>::value) {
-          lay.sput(idx, vr[m][k], vi[m][k]);
-        } else {
-          lay.sre[lay.saddr(idx)] = vr[m][k];
-          lay.sim[lay.saddr(idx)] = vi[m][k];
+        for (int k = 0; k < R; ++k) {
+          const int idx = base + k * NS;
+          if constexpr (IsPairLayout<Layout>::value) {
+            lay.sput(idx, vr[m][k], vi[m][k]);
+          } else {
+            lay.sre[lay.saddr(idx)] = vr[m][k];
+            lay.sim[lay.saddr(idx)] = vi[m][k];
+          }
         }
       }
     }
@@ -1030,8 +1070,37 @@ struct ColsGeom {
   static constexpr int PITCH = C + 1;           // words per element row
   static constexpr int WORDS = L * PITCH;       // per real/imag array
   static constexpr size_t SMEM = 2ull * WORDS * sizeof(T);
+  // later passes: the first stage's table of line powers behind the tile
+  static constexpr size_t super_smem(int first_radix) {
+    return SMEM + (size_t)first_radix * C * sizeof(cplx_t<T>);
+  }
   static constexpr int THREADS = TPL * C;
 };
+
+// Points a thread holds in its widest stage: ceil(L / R / TPL) butterflies.
+template <int L, int TPL, int... Rs>
+__host__ __device__ constexpr int stage_points() {
+  int most = 0;
+  for (int r : {Rs...}) {
+    const int points = (L / r + TPL - 1) / TPL * r;
+    if (points > most) most = points;
+  }
+  return most;
+}
+
+// Resident CTAs a column kernel's registers are capped for: 64 registers for
+// the threads that hold 16 FP32 points (uncapped the later passes took 71 to
+// 79, three CTAs of 256 threads per SM instead of four), 96 up to 24 points,
+// 128 up to 32; twice the points' share for FP64.
+template <typename T, int L, int TPL, int C, int... Rs>
+__host__ __device__ constexpr int cols_min_ctas() {
+  const int points = stage_points<L, TPL, Rs...>();
+  const int regs = sizeof(T) == 4 ? (points <= 16 ? 64 : points <= 24 ? 96 : 128)
+                                  : (points <= 16 ? 128 : points <= 24 ? 168 : 255);
+  const int warps = (TPL * C + 31) / 32;
+  const int ctas = 65536 / (regs * 32 * warps);
+  return ctas < 1 ? 1 : ctas;
+}
 
 // Addressing of this thread's line of a COLS tile (lines j0 .. j0+C-1 of
 // batch entry b).
@@ -1039,12 +1108,12 @@ template <typename T, int L, int TPL, int C, bool TW, class Layout>
 __device__ __forceinline__ void cols_layout(Layout& lay, const ColsArgs<T>& a, long long b,
                                             long long j0, T* sre, T* sim) {
   using G = ColsGeom<T, L, TPL, C>;
-  const long long lines_total = a.total / L;            // M / L
+  const long long lines_total = a.total / L;            // M / L, below 2^32 (L >= 16)
   const int c = threadIdx.x % C;
   const long long j = j0 + c;
-  const long long ns = a.ns_outer;
-  const long long jq = j / ns;
-  const long long jm = j - jq * ns;
+  const unsigned ns = (unsigned)a.ns_outer;             // divides M / L
+  const unsigned jq = TW ? (unsigned)j / ns : 0u;
+  const unsigned jm = (unsigned)j - jq * ns;
   lay.sre = sre;
   lay.sim = sim;
   lay.c = c;
@@ -1052,7 +1121,7 @@ __device__ __forceinline__ void cols_layout(Layout& lay, const ColsArgs<T>& a, l
   cplx_t<T>* out_b = batch_out<T>(a.out, a.out_dist, a.out_table, b);
   lay.gin = in_b + j;
   lay.in_stride = lines_total;
-  lay.gout = out_b + jq * ns * L + jm;
+  lay.gout = out_b + (long long)jq * ns * L + jm;
   lay.out_stride = ns;
   lay.sign_in = a.sign_in;
   lay.sign_out = a.sign_out;
@@ -1065,8 +1134,10 @@ __device__ __forceinline__ void cols_layout(Layout& lay, const ColsArgs<T>& a, l
 }
 
 // Body of one COLS tile: lines j0 .. j0+C-1 of batch entry b, run by threads
-// 0 .. TPL*C-1 of the CTA (every thread of the CTA must call it).
-template <typename T, int L, int TPL, int C, int... Rs>
+// 0 .. TPL*C-1 of the CTA (every thread of the CTA must call it).  HEAD: the
+// first pass (Ns_outer == 1), which has no super-stage twiddles; a kernel of
+// its own, since both in one kernel take the registers of the later passes.
+template <typename T, int L, int TPL, int C, bool HEAD, int... Rs>
 __device__ __forceinline__ void cols_body(const ColsArgs<T>& a, long long b,
                                           long long j0, unsigned char* smem_raw) {
   static_assert(StageProduct<L, Rs...>::value == L, "radices must multiply to L");
@@ -1074,7 +1145,7 @@ __device__ __forceinline__ void cols_body(const ColsArgs<T>& a, long long b,
   T* sre = reinterpret_cast<T*>(smem_raw);
   T* sim = sre + G::WORDS;
   const int t = threadIdx.x / C;
-  if (a.ns_outer == 1) {
+  if constexpr (HEAD) {
     ColsLayout<T, C, G::PITCH, false> lay;
     cols_layout<T, L, TPL, C, false>(lay, a, b, j0, sre, sim);
     StageRunner<T, L, TPL, 1, 0, false, true, true, true, Rs...>::run(lay, t, a.tw);
@@ -1091,6 +1162,7 @@ __device__ __forceinline__ void cols_body(const ColsArgs<T>& a, long long b,
   } else {
     ColsLayout<T, C, G::PITCH, true> lay;
     cols_layout<T, L, TPL, C, true>(lay, a, b, j0, sre, sim);
+    lay.sw = reinterpret_cast<cplx_t<T>*>(smem_raw + G::SMEM);
     StageRunner<T, L, TPL, 1, 0, false, false, true, true, Rs...>::run(lay, t, a.tw);
   }
 }
@@ -1117,14 +1189,14 @@ struct ColsPairLayout : ColsLayout<T, C, PITCH, TW> {
   }
 };
 
-template <typename T, int L, int TPL, int C, int... Rs>
+template <typename T, int L, int TPL, int C, bool HEAD, int... Rs>
 __device__ __forceinline__ void cols_body_pair(const ColsArgs<T>& a, long long b,
                                                long long j0, unsigned char* smem_raw) {
   static_assert(StageProduct<L, Rs...>::value == L, "radices must multiply to L");
   using G = ColsGeom<T, L, TPL, C>;
   cplx_t<T>* sp = reinterpret_cast<cplx_t<T>*>(smem_raw);
   const int t = threadIdx.x / C;
-  if (a.ns_outer == 1) {
+  if constexpr (HEAD) {
     ColsPairLayout<T, C, G::PITCH, false> lay;
     cols_layout<T, L, TPL, C, false>(lay, a, b, j0, nullptr, nullptr);
     lay.sp = sp;
@@ -1142,28 +1214,37 @@ __device__ __forceinline__ void cols_body_pair(const ColsArgs<T>& a, long long b
     ColsPairLayout<T, C, G::PITCH, true> lay;
     cols_layout<T, L, TPL, C, true>(lay, a, b, j0, nullptr, nullptr);
     lay.sp = sp;
+    lay.sw = reinterpret_cast<cplx_t<T>*>(smem_raw + G::SMEM);
     StageRunner<T, L, TPL, 1, 0, false, false, true, true, Rs...>::run(lay, t, a.tw);
   }
 }
 
-template <typename T, int L, int TPL, int C, int... Rs>
-__global__ void __launch_bounds__(TPL * C)
-cols_kernel_pair(const ColsArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const long long groups = (a.total / L) / C;
-  const long long b = blockIdx.x / groups;
-  const long long j0 = (blockIdx.x - b * groups) * C;
-  cols_body_pair<T, L, TPL, C, Rs...>(a, b, j0, smem_raw);
+// Tile of this CTA; the tiles of one transform are below 2^32, so the index
+// split is one 32-bit division.
+template <int L, int C, typename T>
+__device__ __forceinline__ void cols_tile(const ColsArgs<T>& a, long long& b, long long& j0) {
+  const unsigned groups = (unsigned)((a.total / L) / C);   // C divides M/L
+  const unsigned q = blockIdx.x / groups;
+  b = q;
+  j0 = (long long)(blockIdx.x - q * groups) * C;
 }
 
-template <typename T, int L, int TPL, int C, int... Rs>
-__global__ void __launch_bounds__(TPL * C)
+template <typename T, int L, int TPL, int C, bool HEAD, int... Rs>
+__global__ void __launch_bounds__(TPL * C, (cols_min_ctas<T, L, TPL, C, Rs...>()))
+cols_kernel_pair(const ColsArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  long long b, j0;
+  cols_tile<L, C>(a, b, j0);
+  cols_body_pair<T, L, TPL, C, HEAD, Rs...>(a, b, j0, smem_raw);
+}
+
+template <typename T, int L, int TPL, int C, bool HEAD, int... Rs>
+__global__ void __launch_bounds__(TPL * C, (cols_min_ctas<T, L, TPL, C, Rs...>()))
 cols_kernel(const ColsArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const long long groups = (a.total / L) / C;           // C divides M/L
-  const long long b = blockIdx.x / groups;
-  const long long j0 = (blockIdx.x - b * groups) * C;
-  cols_body<T, L, TPL, C, Rs...>(a, b, j0, smem_raw);
+  long long b, j0;
+  cols_tile<L, C>(a, b, j0);
+  cols_body<T, L, TPL, C, HEAD, Rs...>(a, b, j0, smem_raw);
 }
 
 // ---------------------------------------------------------------------------

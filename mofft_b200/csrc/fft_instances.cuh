@@ -14,6 +14,7 @@ struct Entry {
   mofft_kernel_desc desc;
   launch_fn launch;
   func_fn func;
+  func_fn func_tail;      // column passes after the first (null: none)
   // kernels with a constant table of their own (e.g. DFT-matrix operands):
   // its size and its host-side construction; 0 / null for the others
   size_t aux_bytes;
@@ -136,12 +137,21 @@ struct RowsInst {
   }
 };
 
-template <typename T, int L, int TPL, int C, int... Rs>
+// PAIR: exchanges move {re, im} pairs (cols_kernel_pair).
+template <typename T, int L, int TPL, int C, bool PAIR, int... Rs>
 struct ColsInst {
   using G = ColsGeom<T, L, TPL, C>;
-  static const void *func() {
-    return reinterpret_cast<const void *>(&cols_kernel<T, L, TPL, C, Rs...>);
+  static constexpr int kRadices[] = {Rs...};
+  static constexpr size_t kSmemTail = G::super_smem(kRadices[0]);
+  static_assert(kSmemTail <= 227 * 1024, "shared memory of one CTA");
+  using Kernel = void (*)(const ColsArgs<T>);
+  template <bool HEAD>
+  static Kernel kernel() {
+    if constexpr (PAIR) return &cols_kernel_pair<T, L, TPL, C, HEAD, Rs...>;
+    else return &cols_kernel<T, L, TPL, C, HEAD, Rs...>;
   }
+  static const void *func() { return reinterpret_cast<const void *>(kernel<true>()); }
+  static const void *func_tail() { return reinterpret_cast<const void *>(kernel<false>()); }
   static cudaError_t launch(const mofft_pass_args *p, cudaStream_t s) {
     if (p->total % L != 0 || (p->total / L) % C != 0) return cudaErrorInvalidValue;
     if (p->ns_outer != 1 && p->ns_outer % C != 0) return cudaErrorInvalidValue;
@@ -149,8 +159,9 @@ struct ColsInst {
     const long long grid = groups * p->batch;
     if (grid <= 0) return cudaSuccess;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    cols_kernel<T, L, TPL, C, Rs...>
-        <<<(unsigned)grid, G::THREADS, G::SMEM, s>>>(cols_args<T>(p));
+    const bool head = p->ns_outer == 1;
+    const Kernel k = head ? kernel<true>() : kernel<false>();
+    k<<<(unsigned)grid, G::THREADS, head ? G::SMEM : kSmemTail, s>>>(cols_args<T>(p));
     return cudaGetLastError();
   }
   static Entry entry(const char *name) {
@@ -165,46 +176,10 @@ struct ColsInst {
     const int rs[] = {Rs...};
     e.desc.radix_count = (int)sizeof...(Rs);
     for (int i = 0; i < 8; ++i) e.desc.radices[i] = i < (int)sizeof...(Rs) ? rs[i] : 0;
-    e.desc.smem_bytes = G::SMEM;
+    e.desc.smem_bytes = kSmemTail;
     e.launch = &launch;
     e.func = &func;
-    return e;
-  }
-};
-
-// Column pass whose exchanges move {re, im} pairs (cols_kernel_pair).
-template <typename T, int L, int TPL, int C, int... Rs>
-struct ColsPairInst {
-  using G = ColsGeom<T, L, TPL, C>;
-  static const void *func() {
-    return reinterpret_cast<const void *>(&cols_kernel_pair<T, L, TPL, C, Rs...>);
-  }
-  static cudaError_t launch(const mofft_pass_args *p, cudaStream_t s) {
-    if (p->total % L != 0 || (p->total / L) % C != 0) return cudaErrorInvalidValue;
-    if (p->ns_outer != 1 && p->ns_outer % C != 0) return cudaErrorInvalidValue;
-    const long long groups = (p->total / L) / C;
-    const long long grid = groups * p->batch;
-    if (grid <= 0) return cudaSuccess;
-    if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    cols_kernel_pair<T, L, TPL, C, Rs...>
-        <<<(unsigned)grid, G::THREADS, G::SMEM, s>>>(cols_args<T>(p));
-    return cudaGetLastError();
-  }
-  static Entry entry(const char *name) {
-    Entry e{};
-    e.desc.name = name;
-    e.desc.precision_bits = sizeof(T) == 4 ? 32 : 64;
-    e.desc.kind = MOFFT_KERNEL_COLS;
-    e.desc.length = L;
-    e.desc.lines = C;
-    e.desc.threads = G::THREADS;
-    e.desc.staged = 0;
-    const int rs[] = {Rs...};
-    e.desc.radix_count = (int)sizeof...(Rs);
-    for (int i = 0; i < 8; ++i) e.desc.radices[i] = i < (int)sizeof...(Rs) ? rs[i] : 0;
-    e.desc.smem_bytes = G::SMEM;
-    e.launch = &launch;
-    e.func = &func;
+    e.func_tail = &func_tail;
     return e;
   }
 };
@@ -336,9 +311,9 @@ struct GenericInst {
   RowsInst<T, L, TPL, 1, kDerivedTw | kSplitX | kPrefetch | kTwoCtas, __VA_ARGS__>::entry( \
       "rows_" #T "_" #L "_t" #TPL "_b1_sfalse_dxp2")
 #define COLS(T, L, TPL, C, ...) \
-  ColsInst<T, L, TPL, C, __VA_ARGS__>::entry("cols_" #T "_" #L "_t" #TPL "_c" #C)
+  ColsInst<T, L, TPL, C, false, __VA_ARGS__>::entry("cols_" #T "_" #L "_t" #TPL "_c" #C)
 #define COLSP(T, L, TPL, C, ...) \
-  ColsPairInst<T, L, TPL, C, __VA_ARGS__>::entry("cols_" #T "_" #L "_t" #TPL "_c" #C "_p")
+  ColsInst<T, L, TPL, C, true, __VA_ARGS__>::entry("cols_" #T "_" #L "_t" #TPL "_c" #C "_p")
 
 // Each instance file defines one of these.
 const Entry *entries_generic(int *count);

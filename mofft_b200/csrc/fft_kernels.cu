@@ -52,6 +52,9 @@ extern "C" int mofft_cuda_prepare_device(void) {
     if (smem > 227 * 1024) smem = 227 * 1024;
     cudaError_t err = cudaFuncSetAttribute(
         e.func(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err == cudaSuccess && e.func_tail)
+      err = cudaFuncSetAttribute(e.func_tail(),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
   }
   cudaError_t err = rt_prepare_f32();

@@ -93,6 +93,10 @@ mofft_status mofft_search_best(mofft_core **out, int precision_bits,
  * kernel instances as registry indices (-1 = none). */
 int mofft_wisdom_lookup(size_t length, int precision_bits, int *chain,
                         int capacity, int *preferred);
+/* The fastest two-pass schedule of a length whose tuned one has three passes,
+ * for plans without a batch-sized workspace; returns as mofft_wisdom_lookup. */
+int mofft_wisdom_lookup_two_pass(size_t length, int precision_bits, int *chain,
+                                 int capacity, int *preferred);
 
 /* Kernel banks (the reference's compiled code families, portfolio.py:31-35):
  * 0 the specialised kernels with the default codelets (runtime-stage kernels

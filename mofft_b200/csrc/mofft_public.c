@@ -119,8 +119,8 @@ static mofft_status create_with_options(mofft_core **out, int precision_bits,
   /* A tuned schedule never costs memory the untuned one does not: a
    * schedule of three or more passes, or of two passes in place, needs a
    * batch-sized workspace; when the tuned schedule needs one and the model
-   * schedule does not, the plan keeps the model schedule (unless the caller
-   * insists on wisdom). */
+   * schedule does not, the plan takes the tuned two-pass schedule of the
+   * length, else the model's (unless the caller insists on wisdom). */
   if (wisdom && !(options.flags & MOFFT_PLAN_STRICT_WISDOM)) {
     int tuned_passes = 0;
     while (tuned_passes < MOFFT_MAX_PASSES && preferred[tuned_passes] >= 0) ++tuned_passes;
@@ -130,7 +130,9 @@ static mofft_status create_with_options(mofft_core **out, int precision_bits,
         mofft_schedule_preview(precision_bits, length, NULL, 0, 0, &model, NULL, NULL) ==
             MOFFT_SUCCESS &&
         !(model.pass_count >= 3 || (model.pass_count == 2 && in_place)))
-      wisdom = 0;
+      wisdom = in_place ? 0
+                        : mofft_wisdom_lookup_two_pass(length, precision_bits, chain,
+                                                       MOFFT_MAX_STAGES, preferred);
   }
   status = mofft_core_create_tuned(out, precision_bits, length, batch, distance,
                                    direction, placement, wisdom ? chain : NULL,

@@ -15,12 +15,12 @@ static int kernel_index_by_name(const char *name) {
   return -1;
 }
 
-int mofft_wisdom_lookup(size_t length, int precision_bits, int *chain,
-                        int capacity, int *preferred) {
+static int lookup(const mofft_wisdom_entry *table, int entries, size_t length,
+                  int precision_bits, int *chain, int capacity, int *preferred) {
   if (preferred)
     for (int p = 0; p < MOFFT_MAX_PASSES; ++p) preferred[p] = -1;
-  for (int i = 0; i < MOFFT_WISDOM_COUNT; ++i) {
-    const mofft_wisdom_entry *e = &k_mofft_wisdom[i];
+  for (int i = 0; i < entries; ++i) {
+    const mofft_wisdom_entry *e = &table[i];
     if (e->length == length && e->precision_bits == precision_bits &&
         e->count <= capacity) {
       memcpy(chain, e->chain, (size_t)e->count * sizeof(int));
@@ -30,6 +30,18 @@ int mofft_wisdom_lookup(size_t length, int precision_bits, int *chain,
     }
   }
   return 0;
+}
+
+int mofft_wisdom_lookup(size_t length, int precision_bits, int *chain,
+                        int capacity, int *preferred) {
+  return lookup(k_mofft_wisdom, MOFFT_WISDOM_COUNT, length, precision_bits, chain, capacity,
+                preferred);
+}
+
+int mofft_wisdom_lookup_two_pass(size_t length, int precision_bits, int *chain,
+                                 int capacity, int *preferred) {
+  return lookup(k_mofft_wisdom_two_pass, MOFFT_WISDOM_TWO_PASS_COUNT, length, precision_bits,
+                chain, capacity, preferred);
 }
 
 int mofft_wisdom_is_formal(void) { return MOFFT_WISDOM_FORMAL; }

@@ -128,14 +128,17 @@ extern "C" mofft_status mofft_execute_fixed_scratch_f32(
 
   // Only two-pass schedules need the intermediate array this entry point
   // provides.  The tuned schedule of the compiled wisdom runs when it has two
-  // passes (the same kernels an out-of-place PRETUNED plan runs); otherwise
-  // the model's schedule runs when it has two (a tuned three-pass schedule
-  // would need a second intermediate array).
+  // passes (the same kernels an out-of-place PRETUNED plan runs), the tuned
+  // two-pass schedule of the length when it has three (which would need a
+  // second intermediate array); otherwise the model's schedule runs when it
+  // has two.
   int chain[MOFFT_MAX_STAGES];
   int preferred[MOFFT_MAX_PASSES];
   mofft_schedule sched;
   sched.pass_count = 0;
-  const int tuned = mofft_wisdom_lookup(length, 32, chain, MOFFT_MAX_STAGES, preferred);
+  int tuned = mofft_wisdom_lookup(length, 32, chain, MOFFT_MAX_STAGES, preferred);
+  if (tuned > 0 && MOFFT_MAX_PASSES > 2 && preferred[2] >= 0)
+    tuned = mofft_wisdom_lookup_two_pass(length, 32, chain, MOFFT_MAX_STAGES, preferred);
   if (tuned > 0 && preferred[0] >= 0 && preferred[1] >= 0 &&
       (MOFFT_MAX_PASSES < 3 || preferred[2] < 0)) {
     if (!mofft_group_chain_preferred(32, 0, chain, tuned, (long long)length, preferred,

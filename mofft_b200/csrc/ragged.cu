@@ -119,7 +119,7 @@ constexpr int kArgCount = (int)sizeof...(R);
    2ull * (kThreads / TPL) * pair_pitch<float>(L, TPL, kThreads / TPL) * sizeof(float)},
 #define MOFFT_COLS_INFO(ID, L, TPL, ...)                             \
   {ID, L, TPL, 1, kArgCount<__VA_ARGS__>, {__VA_ARGS__},             \
-   ColsGeom<float, L, TPL, kColsLines>::SMEM},
+   ColsGeom<float, L, TPL, kColsLines>::super_smem(16)},
 
 const ConfigInfo kConfigs[] = {MOFFT_RAGGED_ROWS(MOFFT_ROWS_INFO) MOFFT_RAGGED_COLS(MOFFT_COLS_INFO)};
 
@@ -185,8 +185,12 @@ __device__ __forceinline__ ColsArgs<float> cols_args_of(const RItem &it, int pas
   __device__ __noinline__ void tile_##ID(const RItem *__restrict__ itp, int pass,    \
                                          long long b, long long j0,                   \
                                          unsigned char *smem) {                       \
-    cols_body_pair<float, L, TPL, kColsLines, __VA_ARGS__>(cols_args_of(*itp, pass), b, j0, \
-                                                      smem);                          \
+    if (pass == 0)                                                                   \
+      cols_body_pair<float, L, TPL, kColsLines, true, __VA_ARGS__>(                   \
+          cols_args_of(*itp, pass), b, j0, smem);                                     \
+    else                                                                             \
+      cols_body_pair<float, L, TPL, kColsLines, false, __VA_ARGS__>(                  \
+          cols_args_of(*itp, pass), b, j0, smem);                                     \
   }
 MOFFT_RAGGED_ROWS(MOFFT_ROWS_FN)
 MOFFT_RAGGED_COLS(MOFFT_COLS_FN)

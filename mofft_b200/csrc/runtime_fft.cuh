@@ -141,7 +141,6 @@ __device__ __forceinline__ void rt_stage(const RtIo<T>& io, cplx_t<T>* sp, const
         vr[r] = v.x;
         vi[r] = v.y * io.sign;
       }
-      super(vr, vi);
     } else {
       const cplx_t<T>* p = sp + io.src;
 #pragma unroll
@@ -151,14 +150,21 @@ __device__ __forceinline__ void rt_stage(const RtIo<T>& io, cplx_t<T>* sp, const
         vi[r] = v.y;
       }
     }
-    if constexpr (TW) rt_twiddle<T, R>(vr, vi, io.tw, io.ns);
-    Dft<R>::fwd(vr, vi);
   } else {
     // defined on every path: a register that is only written under `act` and
     // read under it behind the barrier counts as live around the stage loop,
     // for every radix at once (the radix-8 class spilled 350 bytes a thread)
 #pragma unroll
     for (int r = 0; r < R; ++r) vr[r] = vi[r] = T(0);
+  }
+  if constexpr (Super::kActive) {
+    super.template fill<R>();
+    __syncthreads();
+  }
+  if (io.act) {
+    if constexpr (Super::kActive) super.template apply<R>(vr, vi);
+    if constexpr (TW) rt_twiddle<T, R>(vr, vi, io.tw, io.ns);
+    Dft<R>::fwd(vr, vi);
   }
   if constexpr (SRC == kShared && DST == kShared) __syncthreads();
   if (io.act) {
@@ -176,18 +182,42 @@ __device__ __forceinline__ void rt_stage(const RtIo<T>& io, cplx_t<T>* sp, const
 }
 
 struct RtNoSuper {
-  template <typename T, int R>
-  __device__ __forceinline__ void operator()(T (&)[R], T (&)[R]) const {}
+  static constexpr bool kActive = false;
 };
 
-// Super-stage twiddle of a later column pass (ColsLayout's table form).
+// Super-stage twiddle of a later column pass: v[r] *= b u^r with b =
+// W^{jmod j} looked up by each thread and the powers u^r of the tile's lines
+// in a table (ColsLayout's scheme; here a line's jmod may wrap inside a tile).
 template <typename T>
 struct RtSuper {
-  ColsLayout<T, 1, 1, true> lay;
-  int j, bf;
+  static constexpr bool kActive = true;
+  ColsLayout<T, 1, 1, true> lay;   // the two-level table, this thread's jmod
+  cplx_t<T>* table;                // radix x lines
+  int j, bf, j0, line, line_shift;
+  unsigned ns;
   template <int R>
-  __device__ __forceinline__ void operator()(T (&vr)[R], T (&vi)[R]) const {
-    lay.template super_twiddle<R>(j, bf, vr, vi);
+  __device__ __forceinline__ void fill() const {
+    ColsLayout<T, 1, 1, true> l = lay;
+    const int lines = 1 << line_shift;
+    for (int q = threadIdx.x; q < R << line_shift; q += blockDim.x) {
+      l.jmod = (unsigned)(j0 + (q & (lines - 1))) % ns;
+      T wr, wi;
+      l.super_w((unsigned)((q >> line_shift) * bf), wr, wi);
+      st_global<T>(table + q, wr, wi);
+    }
+  }
+  template <int R>
+  __device__ __forceinline__ void apply(T (&vr)[R], T (&vi)[R]) const {
+    T br, bi;
+    lay.super_w((unsigned)j, br, bi);
+    cmul<T>(vr[0], vi[0], br, bi);
+#pragma unroll
+    for (int r = 1; r < R; ++r) {
+      const cplx_t<T> u = table[(r << line_shift) + line];
+      T xr = u.x, xi = u.y;
+      cmul<T>(xr, xi, br, bi);
+      cmul<T>(vr[r], vi[r], xr, xi);
+    }
   }
 };
 
@@ -307,8 +337,13 @@ __global__ void __launch_bounds__(MAXT, 1) rt_kernel(const __grid_constant__ RtA
         super.lay.tw_lo = a.tw_lo;
         super.lay.split_shift = a.split_shift;
         super.lay.jmod = (unsigned)(j0 + line) % (unsigned)a.ns_outer;
+        super.table = sp + L * a.pitch;
         super.j = j;
         super.bf = s.bf;
+        super.j0 = j0;
+        super.line = line;
+        super.line_shift = a.line_shift;
+        super.ns = (unsigned)a.ns_outer;
         rt_dispatch<T, MAXR, kGlobal, kShared, false>(s.radix, io, sp, super);
       }
     }

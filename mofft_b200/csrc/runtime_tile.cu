@@ -45,14 +45,16 @@ bool rt_shape(int precision_bits, bool cols, int length, const int *chain, int c
     // exceeds the threads or half an SM's shared memory (runs of 64 bytes
     // still), or while the launch leaves SMs without a CTA
     int c = row;
+    // tile rows of c + 1 pairs, and the first stage's table of line powers
+    auto bytes = [&](int n) { return ((size_t)length * (n + 1) + (size_t)chain[0] * n) * cb; };
     const size_t half = kSmemLimit / 2;
-    while (c > 1 && (c * bf > cap || (size_t)length * (c + 1) * cb > kSmemLimit)) c /= 2;
-    while (c > row / 2 && (c * bf > 512 || (size_t)length * (c + 1) * cb > half)) c /= 2;
+    while (c > 1 && (c * bf > cap || bytes(c) > kSmemLimit)) c /= 2;
+    while (c > row / 2 && (c * bf > 512 || bytes(c) > half)) c /= 2;
     while (c > row / 4 && (line_units + c - 1) / c * (units / line_units) < kSms) c /= 2;
-    if (c < 1 || (size_t)length * (c + 1) * cb > kSmemLimit) return false;
+    if (c < 1 || bytes(c) > kSmemLimit) return false;
     s.lines = c;
     s.pitch = c + 1;
-    s.smem = (size_t)length * s.pitch * cb;
+    s.smem = bytes(c);
     s.threads = (c * bf + 31) / 32 * 32;
     *out = s;
     return true;
