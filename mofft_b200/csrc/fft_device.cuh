@@ -79,6 +79,20 @@ __device__ __forceinline__ void cmul(T& xr, T& xi, T wr, T wi) {
 template <typename T>
 __device__ __forceinline__ cplx_t<T> ld_global(const cplx_t<T>* p) { return __ldcg(p); }
 
+// Programmatic dependent launch.  A pass is launched while the stream's
+// previous kernel still drains: its CTAs may become resident once every CTA
+// of that kernel has started, and wait here until it has completed and its
+// writes are visible.  Nothing before this call touches global memory; the
+// returned pointer (through which the pass reads) carries the order.  The
+// first instruction lets the next pass of the stream start in the same way.
+// Saves the gap between dependent kernels (about 1 us of each launch).
+template <class P>
+__device__ __forceinline__ P* after_previous(P* p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
+  return p;
+}
+
 template <typename T>
 __device__ __forceinline__ void st_global(cplx_t<T>* p, T re, T im) {
   cplx_t<T> v;
@@ -866,16 +880,20 @@ __device__ __forceinline__ void rows_body(const RowsArgs<T>& a, long long b0,
 
 template <typename T, int L, int TPL, int TB, int FLAGS, int... Rs>
 __global__ void __launch_bounds__(TPL * TB)
-rows_kernel(const RowsArgs<T> a) {
+rows_kernel(const RowsArgs<T> args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  RowsArgs<T> a = args;
+  a.in = after_previous(args.in);
   rows_body<T, L, TPL, TB, FLAGS, Rs...>(a, (long long)blockIdx.x * TB, smem_raw);
 }
 
 // The same with registers capped for two resident CTAs per SM (kTwoCtas).
 template <typename T, int L, int TPL, int TB, int FLAGS, int... Rs>
 __global__ void __launch_bounds__(TPL * TB, 2)
-rows_kernel_2cta(const RowsArgs<T> a) {
+rows_kernel_2cta(const RowsArgs<T> args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  RowsArgs<T> a = args;
+  a.in = after_previous(args.in);
   rows_body<T, L, TPL, TB, FLAGS, Rs...>(a, (long long)blockIdx.x * TB, smem_raw);
 }
 
@@ -1033,8 +1051,10 @@ __device__ __forceinline__ void rows_prefetch_body(const RowsArgs<T>& a, unsigne
 
 template <typename T, int L, int TPL, int FLAGS, int... Rs>
 __global__ void __launch_bounds__(TPL, (FLAGS & kTwoCtas) ? 2 : 1)
-rows_prefetch_kernel(const RowsArgs<T> a) {
+rows_prefetch_kernel(const RowsArgs<T> args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  RowsArgs<T> a = args;
+  a.in = after_previous(args.in);
   rows_prefetch_body<T, L, TPL, FLAGS, Rs...>(a, smem_raw);
 }
 
@@ -1231,8 +1251,10 @@ __device__ __forceinline__ void cols_tile(const ColsArgs<T>& a, long long& b, lo
 
 template <typename T, int L, int TPL, int C, bool HEAD, int... Rs>
 __global__ void __launch_bounds__(TPL * C, (cols_min_ctas<T, L, TPL, C, Rs...>()))
-cols_kernel_pair(const ColsArgs<T> a) {
+cols_kernel_pair(const ColsArgs<T> args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  ColsArgs<T> a = args;
+  a.in = after_previous(args.in);
   long long b, j0;
   cols_tile<L, C>(a, b, j0);
   cols_body_pair<T, L, TPL, C, HEAD, Rs...>(a, b, j0, smem_raw);
@@ -1240,8 +1262,10 @@ cols_kernel_pair(const ColsArgs<T> a) {
 
 template <typename T, int L, int TPL, int C, bool HEAD, int... Rs>
 __global__ void __launch_bounds__(TPL * C, (cols_min_ctas<T, L, TPL, C, Rs...>()))
-cols_kernel(const ColsArgs<T> a) {
+cols_kernel(const ColsArgs<T> args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  ColsArgs<T> a = args;
+  a.in = after_previous(args.in);
   long long b, j0;
   cols_tile<L, C>(a, b, j0);
   cols_body<T, L, TPL, C, HEAD, Rs...>(a, b, j0, smem_raw);
@@ -1385,8 +1409,10 @@ __device__ __forceinline__ void generic_dispatch(
 // BANK: the kernel bank whose codelets the stages run (0 default, 1-3 the
 // rewrite families of BankDft).
 template <typename T, bool WIDE, int BANK>
-__global__ void __launch_bounds__(256, WIDE ? 1 : 2) generic_kernel(const GenericArgs<T> a) {
+__global__ void __launch_bounds__(256, WIDE ? 1 : 2) generic_kernel(const GenericArgs<T> args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  GenericArgs<T> a = args;
+  a.in = after_previous(args.in);
   const int L = a.length;
   const bool cols = a.cols != 0;
   const int line_words = cols ? 0 : spad_len<T>(L);

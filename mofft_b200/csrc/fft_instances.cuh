@@ -21,6 +21,26 @@ struct Entry {
   int (*fill_aux)(void *dst);
 };
 
+// One pass kernel on `s`; with p->overlap as a programmatic dependent of the
+// stream's previous kernel (the kernels wait for it themselves,
+// after_previous).
+template <class Args>
+cudaError_t launch_pass(const void *func, unsigned grid, int threads, size_t smem,
+                        const Args &a, const mofft_pass_args *p, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = p->overlap ? 1 : 0;
+  void *params[] = {const_cast<Args *>(&a)};
+  return cudaLaunchKernelExC(&cfg, func, params);
+}
+
 template <typename T>
 RowsArgs<T> rows_args(const mofft_pass_args *p) {
   RowsArgs<T> a;
@@ -102,20 +122,12 @@ struct RowsInst {
       const int resident = persistent_grid();
       if (resident <= 0) return cudaErrorInvalidConfiguration;
       const long long grid = p->batch < resident ? p->batch : resident;
-      rows_prefetch_kernel<T, L, TPL, FLAGS, Rs...>
-          <<<(unsigned)grid, TPL, smem(), s>>>(rows_args<T>(p));
-      return cudaGetLastError();
+      return launch_pass(func(), (unsigned)grid, TPL, smem(), rows_args<T>(p), p, s);
     }
     const long long grid = (p->batch + TB - 1) / TB;
     if (grid <= 0) return cudaSuccess;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    if constexpr ((FLAGS & kTwoCtas) != 0)
-      rows_kernel_2cta<T, L, TPL, TB, FLAGS, Rs...>
-          <<<(unsigned)grid, TPL * TB, smem(), s>>>(rows_args<T>(p));
-    else
-      rows_kernel<T, L, TPL, TB, FLAGS, Rs...>
-          <<<(unsigned)grid, TPL * TB, smem(), s>>>(rows_args<T>(p));
-    return cudaGetLastError();
+    return launch_pass(func(), (unsigned)grid, TPL * TB, smem(), rows_args<T>(p), p, s);
   }
   static Entry entry(const char *name) {
     Entry e{};
@@ -160,9 +172,8 @@ struct ColsInst {
     if (grid <= 0) return cudaSuccess;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const bool head = p->ns_outer == 1;
-    const Kernel k = head ? kernel<true>() : kernel<false>();
-    k<<<(unsigned)grid, G::THREADS, head ? G::SMEM : kSmemTail, s>>>(cols_args<T>(p));
-    return cudaGetLastError();
+    return launch_pass(head ? func() : func_tail(), (unsigned)grid, G::THREADS,
+                       head ? G::SMEM : kSmemTail, cols_args<T>(p), p, s);
   }
   static Entry entry(const char *name) {
     Entry e{};
@@ -250,8 +261,7 @@ struct GenericInst {
     if (grid <= 0) return cudaSuccess;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const size_t smem = generic_smem<T>(p->length, p->lines, p->generic_cols);
-    generic_kernel<T, WIDE, BANK><<<(unsigned)grid, 256, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pass(func(), (unsigned)grid, 256, smem, a, p, s);
   }
   static Entry entry(const char *name) {
     Entry e{};

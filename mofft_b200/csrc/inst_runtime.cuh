@@ -95,9 +95,7 @@ cudaError_t rt_launch(const mofft_pass_args *p, cudaStream_t stream) {
   const int mode = cols ? (a.ns_outer == 1 ? kRtColsHead : kRtColsTail)
                         : (s.staged ? kRtStaged : kRtRows);
   const void *func = rt_func<T>(mode, s.max_radix);
-  void *params[] = {&a};
-  return cudaLaunchKernel(func, dim3((unsigned)grid), dim3((unsigned)s.threads), params, s.smem,
-                          stream);
+  return launch_pass(func, (unsigned)grid, s.threads, s.smem, a, p, stream);
 }
 
 template <typename T>

@@ -1141,6 +1141,7 @@ static mofft_status enqueue_with_work(const mofft_core *c, const void *in, void 
     a.length = ps->length;
     a.lines = ps->lines;
     a.radix_count = ps->radix_count;
+    a.overlap = 1;
     memcpy(a.radices, ps->radices, sizeof(a.radices));
     const int err = mofft_cuda_launch_pass(ps->kernel, &a, stream);
     atomic_fetch_add(&g_launches, 1);

@@ -70,6 +70,8 @@ typedef struct {
    * kernels: the error word their line-copy waits set (may be NULL) */
   const void *aux;
   int *status;
+  int overlap;           /* 1: the launch may overlap the end of the stream's
+                            previous kernel (programmatic dependent launch) */
   int lose_copy;         /* failure check: the kernel's first copy is never
                             issued, so its wait runs out (0 in normal use) */
   /* generic kernel only */

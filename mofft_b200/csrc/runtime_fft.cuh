@@ -243,6 +243,7 @@ __global__ void __launch_bounds__(MAXT, 1) rt_kernel(const __grid_constant__ RtA
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx_t<T>* sp = reinterpret_cast<cplx_t<T>*>(smem_raw);
   constexpr bool COLS = MODE >= kRtColsHead;
+  const cplx_t<T>* const in = after_previous(a.in);
   const int tid = threadIdx.x;
   const int L = a.length;
   const int last = a.stage_count - 1;
@@ -299,7 +300,7 @@ __global__ void __launch_bounds__(MAXT, 1) rt_kernel(const __grid_constant__ RtA
       // the tile's lines as they lie in global memory, kBatch loads in flight
       constexpr int kBatch = sizeof(T) == 4 ? 8 : 4;
       const int points = nl * L;
-      const cplx_t<T>* src = a.in + b * a.in_dist;
+      const cplx_t<T>* src = in + b * a.in_dist;
       for (int q0 = tid; q0 < points; q0 += kBatch * blockDim.x) {
         cplx_t<T> v[kBatch];
 #pragma unroll
@@ -323,11 +324,11 @@ __global__ void __launch_bounds__(MAXT, 1) rt_kernel(const __grid_constant__ RtA
       io.sstep = s.bf;
       rt_dispatch<T, MAXR, kShared, kShared, false>(s.radix, io, sp, RtNoSuper());
     } else if constexpr (MODE == kRtRows) {
-      io.gsrc = a.in + (b + line) * a.in_dist + j;
+      io.gsrc = in + (b + line) * a.in_dist + j;
       io.gsstep = s.bf;
       rt_dispatch<T, MAXR, kGlobal, kShared, false>(s.radix, io, sp, RtNoSuper());
     } else {
-      io.gsrc = a.in + b * a.in_dist + j0 + line + (long long)j * a.total_lines;
+      io.gsrc = in + b * a.in_dist + j0 + line + (long long)j * a.total_lines;
       io.gsstep = (long long)a.total_lines * s.bf;
       if constexpr (MODE == kRtColsHead) {
         rt_dispatch<T, MAXR, kGlobal, kShared, false>(s.radix, io, sp, RtNoSuper());
