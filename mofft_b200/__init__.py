@@ -318,10 +318,12 @@ def _int_array(values: Sequence[int]):
 
 def _pointer_of(buf) -> int:
     """Address of a numpy array or torch tensor (contiguous, complex)."""
-    if hasattr(buf, "data_ptr"):
-        return int(buf.data_ptr())
+    data_ptr = getattr(buf, "data_ptr", None)
+    if data_ptr is not None:
+        return int(data_ptr())
     if hasattr(buf, "ctypes"):
-        return int(buf.ctypes.data)
+        # .ctypes builds a helper object of twice the cost
+        return buf.__array_interface__["data"][0]
     raise TypeError(f"unsupported buffer type {type(buf)!r}")
 
 
@@ -333,6 +335,8 @@ class Plan:
         self.bits = bits
         self._s = "f32" if bits == 32 else "f64"
         self._lib = load()
+        self._execute = self._fn("execute")
+        self._stream: Optional[int] = None
 
     def _fn(self, name: str):
         return getattr(self._lib, f"mofft_{name}_{self._s}")
@@ -372,15 +376,17 @@ class Plan:
 
     def execute(self, inp, out=None) -> None:
         """Run on numpy arrays (host) or torch tensors (device)."""
-        if out is None:
-            out = inp
-        check(self._fn("execute")(self._h, _pointer_of(inp), _pointer_of(out)), "execute")
+        a = _pointer_of(inp)
+        st = self._execute(self._h, a, a if out is None else _pointer_of(out))
+        if st:
+            raise MofftError(st, "execute")
 
     def execute_ptr(self, in_ptr: int, out_ptr: int) -> int:
-        return self._fn("execute")(self._h, in_ptr, out_ptr)
+        return self._execute(self._h, in_ptr, out_ptr)
 
     def set_stream(self, stream_handle: Optional[int]) -> None:
         check(self._fn("plan_set_stream")(self._h, stream_handle or None), "set_stream")
+        self._stream = stream_handle or None
 
     def set_kernel_bank(self, bank: int) -> None:
         check(self._fn("plan_set_kernel_bank")(self._h, bank), "set_kernel_bank")
@@ -557,8 +563,11 @@ def fft(x, direction: int = FORWARD, *, inplace: bool = False):
     batch = x.numel() // n
     bits = 32 if x.dtype == torch.complex64 else 64
     out = x if inplace else torch.empty_like(x)
-    plan = _plan_cache_get(n, batch, direction, inplace, bits, x.device.index or 0)
-    plan.set_stream(torch.cuda.current_stream(x.device).cuda_stream)
+    device = x.get_device()
+    plan = _plan_cache_get(n, batch, direction, inplace, bits, device)
+    stream = torch.cuda.current_stream(device).cuda_stream or None
+    if plan._stream != stream:
+        plan.set_stream(stream)
     plan.execute(x, out)
     return out
 

@@ -21,6 +21,7 @@
  *    for the plan's lifetime.
  */
 #define _GNU_SOURCE
+#include <cuda.h>
 #include <cuda_runtime_api.h>
 #include <errno.h>
 #include <float.h>
@@ -705,6 +706,8 @@ static void release_device(mofft_core *c) {
   if (c->d_work) cudaFree(c->d_work);
   if (c->d_stage[0]) cudaFree(c->d_stage[0]);
   if (c->d_stage[1]) cudaFree(c->d_stage[1]);
+  if (c->h_pinned) cudaFreeHost(c->h_pinned);
+  c->h_pinned = NULL;
   c->d_twiddles = c->d_work = c->d_stage[0] = c->d_stage[1] = NULL;
   c->twiddle_bytes = c->work_bytes = c->stage_bytes = 0;
 }
@@ -1064,7 +1067,34 @@ mofft_status mofft_core_create_tuned(mofft_core **out, int precision_bits,
 /* execute                                                                   */
 /* ------------------------------------------------------------------------ */
 
+typedef CUresult (*pointer_attribute_fn)(void *, CUpointer_attribute, CUdeviceptr);
+
+/* The driver's single-attribute query (cudaPointerGetAttributes collects all
+ * of them at several times the cost), NULL where it cannot be had. */
+static pointer_attribute_fn pointer_attribute(void) {
+  static atomic_uintptr_t cached; /* 0 unknown, 1 unavailable */
+  uintptr_t v = atomic_load_explicit(&cached, memory_order_acquire);
+  if (v == 0) {
+    void *fn = NULL;
+    enum cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found) !=
+            cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      fn = NULL;
+    v = fn ? (uintptr_t)fn : 1;
+    atomic_store_explicit(&cached, v, memory_order_release);
+  }
+  return v == 1 ? NULL : (pointer_attribute_fn)v;
+}
+
 static int is_device_pointer(const void *p) {
+  /* plain device memory is the common answer; everything else (host, managed,
+   * no current context) takes the full query */
+  const pointer_attribute_fn query = pointer_attribute();
+  unsigned int type = 0;
+  if (query && query(&type, CU_POINTER_ATTRIBUTE_MEMORY_TYPE, (CUdeviceptr)p) == CUDA_SUCCESS &&
+      type == CU_MEMORYTYPE_DEVICE)
+    return 1;
   struct cudaPointerAttributes attr;
   if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
     cudaGetLastError();
@@ -1156,9 +1186,9 @@ static mofft_status enqueue_with_work(const mofft_core *c, const void *in, void 
   return MOFFT_SUCCESS;
 }
 
-static mofft_status ensure_staging(mofft_core *c) {
+static mofft_status ensure_staging(mofft_core *c, size_t chunks) {
   const size_t bytes = c->batch * c->distance * mofft_complex_bytes(c->precision_bits);
-  if (!c->stream2 || !c->stream3) {
+  if (chunks > 1 && (!c->stream2 || !c->stream3)) {
     cudaStream_t s2 = (cudaStream_t)c->stream2, s3 = (cudaStream_t)c->stream3;
     if ((!s2 && cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking) != cudaSuccess) ||
         (!s3 && cudaStreamCreateWithFlags(&s3, cudaStreamNonBlocking) != cudaSuccess)) {
@@ -1168,7 +1198,7 @@ static mofft_status ensure_staging(mofft_core *c) {
     c->stream2 = s2;
     c->stream3 = s3;
   }
-  for (int i = 0; i < 64; ++i) {
+  for (size_t i = 0; chunks > 1 && i < chunks; ++i) {
     if (!c->ev_up[i]) {
       cudaEvent_t e;
       if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
@@ -1203,6 +1233,106 @@ static mofft_status ensure_staging(mofft_core *c) {
   return MOFFT_SUCCESS;
 }
 
+/* Largest span of a host-buffer execute that runs on mapped pinned memory.
+ * The kernel then reads and writes the host's memory itself, so a call is two
+ * host copies and one launch: 1024 FP32 points in 19 us instead of 26 with two
+ * pageable transfers around the launch, 16384 points in 34 instead of 54.
+ * Allocating that memory takes 1.3 to 3 ms, some hundred times the saving: a
+ * plan does it at its 32nd such call, so plans that run a few times never pay
+ * it. */
+#define MOFFT_PINNED_SPAN ((size_t)512 << 10)
+#define MOFFT_PINNED_CALLS 32u
+
+/* One-pass schedules without bulk copies of their input (those kernels also
+ * bound waits through an error word). */
+static int runs_on_host_memory(mofft_core *c, size_t span) {
+  if (span > MOFFT_PINNED_SPAN || c->sched.pass_count != 1 || schedule_has_status(c)) return 0;
+  if (c->h_pinned) return 1;
+  if (++c->small_host_calls < MOFFT_PINNED_CALLS) return 0;
+  /* one allocation, input then output; without it the calls stay staged */
+  if (cudaHostAlloc(&c->h_pinned, 2 * MOFFT_PINNED_SPAN, cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    c->h_pinned = NULL;
+    c->small_host_calls = 0;
+    return 0;
+  }
+  return 1;
+}
+
+static mofft_status execute_pinned(mofft_core *c, const void *in, void *out, size_t span) {
+  unsigned char *src = (unsigned char *)c->h_pinned, *dst = src + MOFFT_PINNED_SPAN;
+  const size_t cb = mofft_complex_bytes(c->precision_bits);
+  const size_t line = c->length * cb, pitch = c->distance * cb;
+  memcpy(src, in, span);
+  cudaStream_t run = (cudaStream_t)c->stream;
+  mofft_status st = enqueue_with_work(c, src, dst, c->batch, c->distance, NULL, run);
+  if (cudaStreamSynchronize(run) != cudaSuccess) {
+    cudaGetLastError();
+    st = MOFFT_INTERNAL_ERROR;
+  }
+  if (st != MOFFT_SUCCESS) return st;
+  if (line == pitch) {
+    memcpy(out, dst, span);
+  } else { /* the gaps between transforms stay as they are */
+    for (size_t b = 0; b < c->batch; ++b)
+      memcpy((unsigned char *)out + b * pitch, dst + b * pitch, line);
+  }
+  return MOFFT_SUCCESS;
+}
+
+/* Host buffers (pageable or pinned), c->lock held: staged through plan-owned
+ * memory.  Chunks of about 24 MiB flow through three streams: uploads in order
+ * on one, each chunk's passes on another once its upload has landed, downloads
+ * on a third once its passes are done.  Each copy engine (host to device,
+ * device to host) and the SMs then work back to back, and only real data
+ * dependencies (events) order them.  A single chunk has nothing to overlap and
+ * runs on one stream. */
+static mofft_status execute_host(mofft_core *c, const void *in, void *out) {
+  const size_t cb = mofft_complex_bytes(c->precision_bits);
+  const size_t span = ((c->batch - 1) * c->distance + c->length) * cb;
+  if (runs_on_host_memory(c, span)) return execute_pinned(c, in, out, span);
+  const size_t chunk_bytes = (size_t)24 << 20;
+  size_t chunks = (span + chunk_bytes - 1) / chunk_bytes;
+  if (chunks > c->batch) chunks = c->batch;
+  if (chunks > 64) chunks = 64;
+  if (chunks < 1) chunks = 1;
+  mofft_status st = ensure_staging(c, chunks);
+  if (st != MOFFT_SUCCESS) return st;
+  cudaStream_t run = (cudaStream_t)c->stream;
+  cudaStream_t up = chunks > 1 ? (cudaStream_t)c->stream2 : run;
+  cudaStream_t down = chunks > 1 ? (cudaStream_t)c->stream3 : run;
+  for (size_t k = 0; k < chunks && st == MOFFT_SUCCESS; ++k) {
+    const size_t b0 = k * c->batch / chunks, b1 = (k + 1) * c->batch / chunks;
+    if (b1 == b0) continue;
+    const size_t off = b0 * c->distance * cb;
+    const size_t bytes = ((b1 - b0 - 1) * c->distance + c->length) * cb;
+    unsigned char *din = (unsigned char *)c->d_stage[0] + off;
+    unsigned char *dout = (unsigned char *)c->d_stage[1] + off;
+    void *work = c->d_work ? (unsigned char *)c->d_work + b0 * c->length * cb : NULL;
+    cudaEvent_t uploaded = (cudaEvent_t)c->ev_up[k], done = (cudaEvent_t)c->ev_done[k];
+    if (cudaMemcpyAsync(din, (const unsigned char *)in + off, bytes, cudaMemcpyHostToDevice,
+                        up) != cudaSuccess ||
+        (up != run && (cudaEventRecord(uploaded, up) != cudaSuccess ||
+                       cudaStreamWaitEvent(run, uploaded, 0) != cudaSuccess)))
+      st = MOFFT_INTERNAL_ERROR;
+    if (st == MOFFT_SUCCESS)
+      st = enqueue_with_work(c, din, dout, b1 - b0, c->distance, work, run);
+    if (st == MOFFT_SUCCESS &&
+        ((down != run && (cudaEventRecord(done, run) != cudaSuccess ||
+                          cudaStreamWaitEvent(down, done, 0) != cudaSuccess)) ||
+         cudaMemcpyAsync((unsigned char *)out + off, dout, bytes, cudaMemcpyDeviceToHost,
+                         down) != cudaSuccess))
+      st = MOFFT_INTERNAL_ERROR;
+  }
+  cudaStream_t streams[3] = {up, run, down};
+  for (int i = chunks > 1 ? 0 : 2; i < 3; ++i)
+    if (cudaStreamSynchronize(streams[i]) != cudaSuccess && st == MOFFT_SUCCESS)
+      st = MOFFT_INTERNAL_ERROR;
+  if (st != MOFFT_SUCCESS) cudaGetLastError();
+  if (st == MOFFT_SUCCESS && schedule_has_status(c)) st = mofft_core_check_status(c);
+  return st;
+}
+
 mofft_status mofft_core_execute(const mofft_core *cc, const void *in, void *out) {
   mofft_core *c = (mofft_core *)cc; /* staging buffers are lazily owned state */
   if (!c || !in || !out) return MOFFT_INVALID_ARGUMENT;
@@ -1230,54 +1360,9 @@ mofft_status mofft_core_execute(const mofft_core *cc, const void *in, void *out)
   } else if (dev_in != dev_out) {
     st = MOFFT_INVALID_ARGUMENT; /* mixed host/device buffers */
   } else {
-    /* host buffers: stage through plan-owned device memory, blocking */
+    /* host buffers, blocking */
     pthread_mutex_lock(&c->lock);
-    st = ensure_staging(c);
-    if (st == MOFFT_SUCCESS) {
-      /* Chunks of about 24 MiB flow through three streams: uploads in order
-       * on one, each chunk's passes on another once its upload has landed,
-       * downloads on a third once its passes are done.  Each copy engine
-       * (host to device, device to host) and the SMs then work back to back,
-       * and only real data dependencies (events) order them. */
-      const size_t cb = mofft_complex_bytes(c->precision_bits);
-      const size_t span = ((c->batch - 1) * c->distance + c->length) * cb;
-      const size_t chunk_bytes = (size_t)24 << 20;
-      size_t chunks = (span + chunk_bytes - 1) / chunk_bytes;
-      if (chunks > c->batch) chunks = c->batch;
-      if (chunks > 64) chunks = 64;
-      if (chunks < 1) chunks = 1;
-      cudaStream_t up = (cudaStream_t)c->stream2, run = (cudaStream_t)c->stream,
-                   down = (cudaStream_t)c->stream3;
-      for (size_t k = 0; k < chunks && st == MOFFT_SUCCESS; ++k) {
-        const size_t b0 = k * c->batch / chunks, b1 = (k + 1) * c->batch / chunks;
-        if (b1 == b0) continue;
-        const size_t off = b0 * c->distance * cb;
-        const size_t bytes = ((b1 - b0 - 1) * c->distance + c->length) * cb;
-        unsigned char *din = (unsigned char *)c->d_stage[0] + off;
-        unsigned char *dout = (unsigned char *)c->d_stage[1] + off;
-        void *work = c->d_work ? (unsigned char *)c->d_work + b0 * c->length * cb : NULL;
-        cudaEvent_t uploaded = (cudaEvent_t)c->ev_up[k], done = (cudaEvent_t)c->ev_done[k];
-        if (cudaMemcpyAsync(din, (const unsigned char *)in + off, bytes,
-                            cudaMemcpyHostToDevice, up) != cudaSuccess ||
-            cudaEventRecord(uploaded, up) != cudaSuccess ||
-            cudaStreamWaitEvent(run, uploaded, 0) != cudaSuccess)
-          st = MOFFT_INTERNAL_ERROR;
-        if (st == MOFFT_SUCCESS)
-          st = enqueue_with_work(c, din, dout, b1 - b0, c->distance, work, run);
-        if (st == MOFFT_SUCCESS &&
-            (cudaEventRecord(done, run) != cudaSuccess ||
-             cudaStreamWaitEvent(down, done, 0) != cudaSuccess ||
-             cudaMemcpyAsync((unsigned char *)out + off, dout, bytes, cudaMemcpyDeviceToHost,
-                             down) != cudaSuccess))
-          st = MOFFT_INTERNAL_ERROR;
-      }
-      cudaStream_t streams[3] = {up, run, down};
-      for (int i = 0; i < 3; ++i)
-        if (cudaStreamSynchronize(streams[i]) != cudaSuccess && st == MOFFT_SUCCESS)
-          st = MOFFT_INTERNAL_ERROR;
-      if (st != MOFFT_SUCCESS) cudaGetLastError();
-      if (st == MOFFT_SUCCESS && schedule_has_status(c)) st = mofft_core_check_status(c);
-    }
+    st = execute_host(c, in, out);
     pthread_mutex_unlock(&c->lock);
   }
   if (saved >= 0 && saved != c->device) cudaSetDevice(saved);

@@ -77,6 +77,9 @@ typedef struct mofft_core {
   void *stream2;           /* second plan-owned stream of the host-buffer
                               pipeline (lazy) */
   size_t stage_bytes;
+  void *h_pinned;          /* small host-buffer executes: mapped pinned input
+                              and output the kernel works on (lazy) */
+  unsigned small_host_calls;
   pthread_mutex_t lock;
   /* MEASURE plans: how the model's order compared with the timings */
   int measured;

@@ -1,0 +1,36 @@
+"""Host-buffer executes: the first calls of a plan are staged, later small ones
+run on mapped pinned memory; both against the oracle, at the limits of that
+path (its call count, its span, gaps between transforms, one-pass only)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import mofft_b200 as m
+import oracle
+from tests.conftest import cuda_available, fp32_tol, fp64_tol, rel_l2
+
+pytestmark = [pytest.mark.gpu,
+              pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")]
+
+CTYPE = {32: np.complex64, 64: np.complex128}
+
+
+@pytest.mark.parametrize("n,batch,gap", [(16, 1, 0), (1000, 3, 5), (1024, 64, 0), (1024, 65, 0),
+                                         (8192, 4, 0), (16384, 1, 0), (32768, 1, 0)])
+@pytest.mark.parametrize("bits", [32, 64])
+def test_repeated_host_executes(n, batch, gap, bits):
+    dist = n + gap
+    tol = fp32_tol(n) if bits == 32 else fp64_tol(n)
+    for placement in (m.OUT_OF_PLACE, m.IN_PLACE):
+        with m.Plan.create(n, m.BACKWARD, placement, bits=bits, batch=batch,
+                           distance=dist) as plan:
+            for call in (1, 31, 32, 33, 40):
+                while getattr(plan, "calls", 0) < call:
+                    plan.calls = getattr(plan, "calls", 0) + 1
+                    buf = oracle.uniform(batch * dist, seed=plan.calls, dtype=CTYPE[bits])
+                    out = buf.copy() if placement == m.IN_PLACE else np.zeros_like(buf)
+                    plan.execute(out if placement == m.IN_PLACE else buf, out)
+                lines = buf.reshape(batch, dist)[:, :n].astype(np.complex128)
+                got = out.reshape(batch, dist)[:, :n]
+                assert rel_l2(got, oracle.fft_ld(lines, m.BACKWARD)) <= tol, (placement, call)
