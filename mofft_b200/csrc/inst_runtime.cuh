@@ -19,28 +19,32 @@ bool rt_pass_shape(const mofft_pass_args *p, RtShape *s) {
                   p->radix_count, line_units * p->batch, line_units, s);
 }
 
-// Smallest register class that holds the chain's largest radix.
+// Smallest register class that holds the chain's largest radix, or the
+// several-butterfly kernels.
 template <typename T, int MODE>
-const void *rt_func(int max_radix) {
+const void *rt_func(int max_radix, bool multi) {
   constexpr int bits = sizeof(T) == 4 ? 32 : 64;
   constexpr bool cols = MODE >= kRtColsHead;
+  if (multi)
+    return reinterpret_cast<const void *>(
+        &rt_kernel<T, MODE, 16, true, rt_max_threads(bits, cols, 16, true)>);
   if (max_radix <= 8)
     return reinterpret_cast<const void *>(
-        &rt_kernel<T, MODE, 8, rt_max_threads(bits, cols, 8)>);
+        &rt_kernel<T, MODE, 8, false, rt_max_threads(bits, cols, 8, false)>);
   if (max_radix <= 11)
     return reinterpret_cast<const void *>(
-        &rt_kernel<T, MODE, 11, rt_max_threads(bits, cols, 11)>);
+        &rt_kernel<T, MODE, 11, false, rt_max_threads(bits, cols, 11, false)>);
   return reinterpret_cast<const void *>(
-      &rt_kernel<T, MODE, 16, rt_max_threads(bits, cols, 16)>);
+      &rt_kernel<T, MODE, 16, false, rt_max_threads(bits, cols, 16, false)>);
 }
 
 template <typename T>
-const void *rt_func(int mode, int max_radix) {
+const void *rt_func(int mode, int max_radix, bool multi) {
   switch (mode) {
-    case kRtRows: return rt_func<T, kRtRows>(max_radix);
-    case kRtStaged: return rt_func<T, kRtStaged>(max_radix);
-    case kRtColsHead: return rt_func<T, kRtColsHead>(max_radix);
-    default: return rt_func<T, kRtColsTail>(max_radix);
+    case kRtRows: return rt_func<T, kRtRows>(max_radix, multi);
+    case kRtStaged: return rt_func<T, kRtStaged>(max_radix, multi);
+    case kRtColsHead: return rt_func<T, kRtColsHead>(max_radix, multi);
+    default: return rt_func<T, kRtColsTail>(max_radix, multi);
   }
 }
 
@@ -94,17 +98,18 @@ cudaError_t rt_launch(const mofft_pass_args *p, cudaStream_t stream) {
   if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const int mode = cols ? (a.ns_outer == 1 ? kRtColsHead : kRtColsTail)
                         : (s.staged ? kRtStaged : kRtRows);
-  const void *func = rt_func<T>(mode, s.max_radix);
+  const void *func = rt_func<T>(mode, s.max_radix, s.multi != 0);
   return launch_pass(func, (unsigned)grid, s.threads, s.smem, a, p, stream);
 }
 
 template <typename T>
 cudaError_t rt_prepare() {
-  const int radix[] = {8, 11, 16};
-  for (int r : radix)
+  const int radix[] = {8, 11, 16, 16};
+  for (int i = 0; i < 4; ++i)
     for (int mode = kRtRows; mode <= kRtColsTail; ++mode) {
-      const cudaError_t err = cudaFuncSetAttribute(
-          rt_func<T>(mode, r), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      const cudaError_t err =
+          cudaFuncSetAttribute(rt_func<T>(mode, radix[i], i == 3),
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
       if (err != cudaSuccess) return err;
     }
   return cudaSuccess;

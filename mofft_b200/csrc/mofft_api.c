@@ -355,11 +355,12 @@ static int make_pass(int precision_bits, unsigned bank, const int *chain,
   }
   const int g = generic_kernel_index(precision_bits, bank, chain + begin, count);
   if (g < 0) return 0;
-  int rt_lines, rt_threads;
+  int rt_lines, rt_threads, rt_ctas;
   size_t rt_smem;
   if (bank == 0 && mofft_cuda_kernel_get(g)->radices[0] <= 16 &&
       mofft_cuda_runtime_tile(precision_bits, !single, (int)length, chain + begin, count,
-                              single ? 1 : total / length, &rt_lines, &rt_threads, &rt_smem)) {
+                              single ? 1 : total / length, &rt_lines, &rt_threads, &rt_smem,
+                              &rt_ctas)) {
     out->kernel = g;
     out->kind = MOFFT_KERNEL_GENERIC;
     out->lines = rt_lines;
@@ -491,27 +492,27 @@ int mofft_auto_radices(long long length, int *out, int capacity) {
 }
 
 /* Cost of a runtime-chain line DFT, in instructions per point: each stage's
- * codelet, an exchange, a barrier and the stage twiddles per stage boundary
- * (about 16), and the registers a tile holds per point (threads = the most
- * butterflies of any stage, each with the largest radix's footprint), which
- * bound the points an SM has in flight. */
+ * codelet, 12 for the exchange, barrier and twiddles of a stage boundary, and a
+ * penalty as the points resident per SM fall below 96 KB.  Fitted to timings of
+ * every chain of 34 lengths (60-10080 points, both precisions, whole transforms
+ * and column passes): the chain it picks takes 2 % longer than the fastest on
+ * average, 1.1 to 1.5 times as long in nine of the 123 cases. */
 static double runtime_chain_cost(int precision_bits, int cols, long long length,
                                  long long line_units, const int *chain, int count) {
-  int lines, threads;
+  int lines, threads, ctas;
   size_t smem;
   if (!mofft_cuda_runtime_tile(precision_bits, cols, (int)length, chain, count, line_units,
-                               &lines, &threads, &smem))
+                               &lines, &threads, &smem, &ctas))
     return 1e6 + count;
-  double cost = 16.0 * (count - 1);
-  int lo = 64, hi = 0;
-  for (int i = 0; i < count; ++i) {
+  double cost = 12.0 * (count - 1);
+  for (int i = 0; i < count; ++i)
     for (int k = 0; k < MOFFT_CODELET_COST_COUNT; ++k)
       if (k_mofft_codelet_costs[k].radix == chain[i])
         cost += (double)k_mofft_codelet_costs[k].instr / chain[i];
-    if (chain[i] < lo) lo = chain[i];
-    if (chain[i] > hi) hi = chain[i];
-  }
-  return cost + (double)(16 + 3 * hi) / lo;
+  const double resident = (double)ctas * lines * (double)length *
+                          (double)mofft_complex_bytes(precision_bits) / 98304.0;
+  if (resident < 1.0) cost += 16.0 * (1.0 / resident - 1.0);
+  return cost;
 }
 
 typedef struct {
@@ -616,6 +617,71 @@ int mofft_model_chain_multipass(int precision_bits, unsigned bank, size_t length
   return model_chain(precision_bits, bank, length, chain, capacity, 0);
 }
 
+typedef struct {
+  int chain[MOFFT_MAX_STAGES];
+  int count;
+  group_score score;
+  double seconds;
+} ranked_split;
+
+/* What a split costs: the device-time model's seconds for compiled kernels and
+ * the rewrite-family banks; for bank 0 splits with runtime-chain passes a cost
+ * per point, fitted to timings of every split of 28 lengths (18000 to 10^6
+ * points, both precisions: the chosen split takes 3.6 % longer than the fastest
+ * on average; the device-time model's choice 10.9 %).  Per pass: its codelets, 8
+ * per stage boundary, a penalty below 64 KB resident per SM and a constant;
+ * runtime-chain passes 1.4 times that. */
+static double split_cost(int precision_bits, unsigned bank, size_t length, size_t batch,
+                         const mofft_schedule *s, int generic) {
+  if (bank != 0 || generic == 0)
+    return mofft_gpu_schedule_seconds(precision_bits, length, batch, s);
+  const double cb = (double)mofft_complex_bytes(precision_bits);
+  double total = 0.0;
+  for (int p = 0; p < s->pass_count; ++p) {
+    const mofft_pass *ps = &s->pass[p];
+    const mofft_kernel_desc *d = mofft_cuda_kernel_get(ps->kernel);
+    int lines = ps->lines, threads, ctas = 1;
+    size_t smem;
+    const int runtime = ps->kind == MOFFT_KERNEL_GENERIC;
+    if (!runtime) {
+      ctas = 65536 / ((precision_bits == 32 ? 64 : 128) * d->threads);
+      if ((size_t)ctas * (d->smem_bytes + 1024) > 228u * 1024u)
+        ctas = (int)(228u * 1024u / (d->smem_bytes + 1024));
+      if (ctas < 1) ctas = 1;
+    } else if (!mofft_cuda_runtime_tile(precision_bits, 1, ps->length, ps->radices,
+                                        ps->radix_count, (long long)length / ps->length, &lines,
+                                        &threads, &smem, &ctas)) {
+      return 1e6;
+    }
+    double cost = 60.0 + 8.0 * (ps->radix_count - 1);
+    for (int i = 0; i < ps->radix_count; ++i)
+      for (int k = 0; k < MOFFT_CODELET_COST_COUNT; ++k)
+        if (k_mofft_codelet_costs[k].radix == ps->radices[i])
+          cost += (double)k_mofft_codelet_costs[k].instr / ps->radices[i];
+    const double resident = (double)ctas * lines * (double)ps->length * cb / 65536.0;
+    if (resident < 1.0) cost += 8.0 * (1.0 / resident - 1.0);
+    total += runtime ? 1.4 * cost : cost;
+  }
+  return total;
+}
+
+static int generic_passes(const mofft_schedule *s) {
+  int n = 0;
+  for (int p = 0; p < s->pass_count; ++p) n += s->pass[p].kind == MOFFT_KERNEL_GENERIC;
+  return n;
+}
+
+/* Fewest passes; compiled kernels throughout before runtime-chain passes (the
+ * two costs have different units); then the cost. */
+static int split_less(const ranked_split *a, const ranked_split *b) {
+  if (a->score.passes != b->score.passes) return a->score.passes < b->score.passes;
+  if ((a->score.generic == 0) != (b->score.generic == 0)) return a->score.generic == 0;
+  if (a->seconds < 1e300 && b->seconds < 1e300 &&
+      fabs(a->seconds - b->seconds) > 1e-3 * b->seconds)
+    return a->seconds < b->seconds;
+  return score_less(&a->score, &b->score);
+}
+
 static int model_chain(int precision_bits, unsigned bank, size_t length, int *chain,
                        int capacity, int one_pass) {
   mofft_schedule sched;
@@ -628,23 +694,22 @@ static int model_chain(int precision_bits, unsigned bank, size_t length, int *ch
                                      (long long)length, &sched) &&
       sched.pass_count == 1)
     return count;
-  /* multi-pass: best balanced split whose passes have kernels */
-  enum { kMaxDiv = 4096 };
+  /* multi-pass: best split whose passes have kernels.  Splits of the fewest
+   * passes are ranked by the device-time model (mofft_gpu_model.c) over a batch
+   * of about 2^25 points, the choice the reference's choose_factorization makes
+   * with its cost model (src/mofft.c:327-351); a split the model cannot price
+   * ranks by the canonical grouping score.  A plan groups its chain
+   * canonically, which may cut it elsewhere than the split it came from, so the
+   * best few splits are priced again as the schedules that result. */
+  enum { kMaxDiv = 4096, kKeep = 6 };
   static __thread long long divs[kMaxDiv];
   int ndiv = 0;
   const long long n = (long long)length;
   collect_divisors(n, 2, 1 << 16, divs, &ndiv, kMaxDiv);
-  int best_count = -1;
-  group_score best = {1 << 30, 1 << 30, 1e300};
-  double best_seconds = 1e300;
-  /* Splits of the fewest passes are ranked by the device-time model
-   * (mofft_gpu_model.c) over a batch of about 2^25 points, the choice the
-   * reference's choose_factorization makes with its cost model
-   * (src/mofft.c:327-351); a split the model cannot price ranks by the
-   * canonical grouping score. */
   const size_t model_batch = n >= (1LL << 25) ? 1 : (size_t)((1LL << 25) / n);
-  int tmp[MOFFT_MAX_STAGES];
-  for (int passes = 2; passes <= 3 && best_count < 0; ++passes) {
+  ranked_split kept[kKeep];
+  int nkept = 0;
+  for (int passes = 2; passes <= 3 && nkept == 0; ++passes) {
     for (int a = 0; a < ndiv; ++a) {
       for (int b = 0; b < (passes == 3 ? ndiv : 1); ++b) {
         long long L[3];
@@ -656,45 +721,47 @@ static int model_chain(int precision_bits, unsigned bank, size_t length, int *ch
           if ((n / L[0]) % L[1] != 0) continue;
           L[2] = n / L[0] / L[1];
         }
-        int total_count = 0;
+        ranked_split c;
+        c.count = 0;
         long long ns = 1;
         int ok = 1;
         int cuts[MOFFT_MAX_PASSES];
         for (int p = 0; p < passes && ok; ++p) {
           if (L[p] < 2 || L[p] > (1 << 16)) { ok = 0; break; }
-          const int c = preferred_chain(precision_bits, bank, MOFFT_KERNEL_COLS,
-                                        L[p], n, ns, tmp + total_count,
-                                        MOFFT_MAX_STAGES - total_count);
-          if (c <= 0) { ok = 0; break; }
-          total_count += c;
-          if (p < passes - 1) cuts[p] = total_count;
+          const int k = preferred_chain(precision_bits, bank, MOFFT_KERNEL_COLS, L[p], n, ns,
+                                        c.chain + c.count, MOFFT_MAX_STAGES - c.count);
+          if (k <= 0) { ok = 0; break; }
+          c.count += k;
+          if (p < passes - 1) cuts[p] = c.count;
           ns *= L[p];
         }
-        if (!ok) continue;
-        group_score score;
-        if (!try_split(precision_bits, bank, tmp, total_count, cuts, passes, n,
-                       NULL, &sched, &score))
+        if (!ok || !try_split(precision_bits, bank, c.chain, c.count, cuts, passes, n, NULL,
+                              &sched, &c.score))
           continue;
-        const double seconds =
-            mofft_gpu_schedule_seconds(precision_bits, (size_t)n, model_batch, &sched);
-        int better;
-        if (best_count < 0 || score.passes != best.passes)
-          better = best_count < 0 || score.passes < best.passes;
-        else if (seconds < 1e300 && best_seconds < 1e300 &&
-                 fabs(seconds - best_seconds) > 1e-3 * best_seconds)
-          better = seconds < best_seconds;
-        else
-          better = score_less(&score, &best);
-        if (better) {
-          best = score;
-          best_seconds = seconds;
-          best_count = total_count;
-          memcpy(chain, tmp, (size_t)total_count * sizeof(int));
-        }
+        c.seconds = split_cost(precision_bits, bank, (size_t)n, model_batch, &sched,
+                               c.score.generic);
+        int at = nkept;
+        while (at > 0 && split_less(&c, &kept[at - 1])) --at;
+        if (at >= kKeep) continue;
+        if (nkept < kKeep) ++nkept;
+        memmove(kept + at + 1, kept + at, (size_t)(nkept - 1 - at) * sizeof(*kept));
+        kept[at] = c;
       }
     }
   }
-  return best_count;
+  int best = -1;
+  for (int i = 0; i < nkept; ++i) {
+    if (!mofft_group_chain(precision_bits, bank, kept[i].chain, kept[i].count, n, &sched))
+      continue;
+    kept[i].score.passes = sched.pass_count;
+    kept[i].score.generic = generic_passes(&sched);
+    kept[i].seconds = split_cost(precision_bits, bank, (size_t)n, model_batch, &sched,
+                                 kept[i].score.generic);
+    if (best < 0 || split_less(&kept[i], &kept[best])) best = i;
+  }
+  if (best < 0) return -1;
+  memcpy(chain, kept[best].chain, (size_t)kept[best].count * sizeof(int));
+  return kept[best].count;
 }
 
 /* ------------------------------------------------------------------------ */

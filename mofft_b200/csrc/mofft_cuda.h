@@ -88,12 +88,12 @@ const mofft_kernel_desc *mofft_cuda_kernel_get(int index);
 size_t mofft_cuda_generic_smem(int precision_bits, int length, int lines,
                                int cols);
 /* Tile of the runtime-chain kernels (runtime_fft.cuh), which run kernel bank
- * 0's narrow generic passes whose chain fits them: lines and threads per CTA
- * and dynamic shared memory; 0 when the chain does not fit.  line_units: lines
+ * 0's narrow generic passes whose chain fits them: lines and threads per CTA,
+ * dynamic shared memory and resident CTAs per SM; 0 when the chain does not fit.  line_units: lines
  * of one transform of a column pass (cols), 1 otherwise. */
 int mofft_cuda_runtime_tile(int precision_bits, int cols, int length,
                             const int *chain, int count, long long line_units,
-                            int *lines, int *threads, size_t *smem);
+                            int *lines, int *threads, size_t *smem, int *ctas);
 /* Opt every kernel into its shared-memory size on the current device.
  * Returns a cudaError_t value (0 = success). */
 int mofft_cuda_prepare_device(void);

@@ -82,14 +82,14 @@ static double pass_seconds(int precision_bits, size_t length, size_t batch,
       (double)(ps->kind == MOFFT_KERNEL_GENERIC ? ps->smem_bytes : d->smem_bytes);
   const double threads = (double)(d->threads > 0 ? d->threads : 256);
   double ctas = floor(GM_THREADS_PER_SM / threads);
-  /* runtime-chain passes: the tile rule's threads, at 64 (128) registers */
-  int rt_lines, rt_threads = 0;
+  /* runtime-chain passes: the tile rule's occupancy */
+  int rt_lines, rt_threads, rt_ctas = 0;
   size_t rt_smem;
   if (ps->kind == MOFFT_KERNEL_GENERIC && d->bank == 0 && d->radices[0] <= 16 &&
       mofft_cuda_runtime_tile(precision_bits, cols, ps->length, ps->radices, ps->radix_count,
                               cols ? (long long)length / ps->length : 1, &rt_lines,
-                              &rt_threads, &rt_smem))
-    ctas = floor((precision_bits == 32 ? 1024.0 : 512.0) / (double)rt_threads);
+                              &rt_threads, &rt_smem, &rt_ctas))
+    ctas = (double)rt_ctas;
   if (smem > 0.0 && GM_SMEM_PER_SM / smem < ctas) ctas = floor(GM_SMEM_PER_SM / smem);
   if (ctas > 32.0) ctas = 32.0;
   if (ctas < 1.0) ctas = 1.0;
@@ -105,7 +105,7 @@ static double pass_seconds(int precision_bits, size_t length, size_t batch,
     if (s > 0 || !first_pass) instr += 5.0; /* twiddle load + complex multiply */
     if (s > 0) instr += 4.0;                /* exchange: store and load re, im */
   }
-  if (ps->kind == MOFFT_KERNEL_GENERIC) instr *= rt_threads > 0 ? 1.4 : 2.0;
+  if (ps->kind == MOFFT_KERNEL_GENERIC) instr *= rt_ctas > 0 ? 1.4 : 2.0;
   if (precision_bits == 64) instr *= 1.6;
   if (ps->kind == MOFFT_KERNEL_TENSOR || ps->kind == MOFFT_KERNEL_TENSOR_COLS) instr *= 0.6;
   const double t_issue = points * instr / (GM_THREAD_INSTR_PER_S * GM_ISSUE_EFF);

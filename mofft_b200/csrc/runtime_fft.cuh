@@ -116,119 +116,196 @@ enum RtMode {
   kRtColsTail = 3   // later pass: super-stage twiddles, strided stores
 };
 
-// One stage's butterfly: gathers from the tile or (SRC == kGlobal) global
-// memory, scatters likewise.
+// Where a butterfly of a stage lies.
 template <typename T>
 struct RtIo {
   bool act;
   int src, sstep, dst, dstep;     // tile addresses, in pairs
-  const cplx_t<T>* gsrc;
-  cplx_t<T>* gdst;
+  const cplx_t<T>* gsrc;          // first stage on global memory
+  cplx_t<T>* gdst;                // last stage on global memory
   long long gsstep, gdstep;
   const cplx_t<T>* tw;            // this butterfly's stage twiddles
-  int ns;
-  T sign;
+  int j, line;
 };
 
-template <typename T, int R, Where SRC, Where DST, bool TW, class Super>
-__device__ __forceinline__ void rt_stage(const RtIo<T>& io, cplx_t<T>* sp, const Super& super) {
-  T vr[R], vi[R];
-  if (io.act) {
-    if constexpr (SRC == kGlobal) {
+// A CTA's tile: which lines, and the place of each butterfly.
+template <typename T, int MODE>
+struct RtTile {
+  static constexpr bool COLS = MODE >= kRtColsHead;
+  const RtArgs<T>& a;
+  const cplx_t<T>* in;
+  long long b;                    // ROWS: first transform; COLS: the transform
+  int j0, nl;                     // COLS: first line; lines inside the batch
+
+  // butterfly w of stage s; only the fields the stage uses are computed
+  template <bool FIRST, bool LAST>
+  __device__ __forceinline__ RtIo<T> at(const RtStage& s, int w) const {
+    RtIo<T> io;
+    if (COLS) {
+      io.line = w & (a.lines - 1);
+      io.j = w >> a.line_shift;
+      io.act = io.j < s.bf && io.line < nl;
+    } else {
+      io.line = rt_div(w, s.magic_bf);
+      io.j = w - io.line * s.bf;
+      io.act = io.line < nl;
+    }
+    const int j = io.j;
+    const int step = COLS ? a.pitch : 1;   // pairs between a line's points
+    const int base = COLS ? io.line : io.line * a.pitch;
+    // first stage: Ns = 1 and the input is not padded; last: Ns R = L
+    const int jq = FIRST ? j : LAST ? 0 : rt_div(j, s.magic_ns);
+    const int jm = FIRST ? 0 : LAST ? j : j - jq * s.ns;
+    io.src = base + (FIRST ? j : j + jq * s.gpad) * step;
+    io.sstep = (FIRST ? s.bf : s.gstep) * step;
+    io.dst = base + (jq * s.sblk + jm) * step;
+    io.dstep = (FIRST ? 1 : s.ns) * step;
+    io.tw = a.tw + s.twoff + jm;
+    if (COLS) {
+      const unsigned ns = (unsigned)a.ns_outer, jl = (unsigned)(j0 + io.line);
+      const unsigned q = MODE == kRtColsTail ? jl / ns : 0u;
+      io.gsrc = in + b * a.in_dist + jl + (long long)j * a.total_lines;
+      io.gsstep = (long long)a.total_lines * s.bf;
+      io.gdst = a.out + b * a.out_dist + (long long)q * ns * a.length + (jl - q * ns) +
+                j * a.ns_outer;
+      io.gdstep = a.ns_outer * s.ns;
+    } else {
+      io.gsrc = in + (b + io.line) * a.in_dist + j;
+      io.gsstep = s.bf;
+      io.gdst = a.out + (b + io.line) * a.out_dist + j;
+      io.gdstep = s.ns;
+    }
+    return io;
+  }
+};
+
+// Super-stage twiddle of a later column pass: v[r] *= b u^r with b =
+// W^{jmod j} looked up by each thread and the powers u^r of the tile's lines
+// in a table behind the tile (ColsLayout's scheme; here a line's jmod may wrap
+// inside a tile).
+template <typename T, int R>
+__device__ __forceinline__ void rt_super_fill(const RtTile<T, kRtColsTail>& tile, int bf,
+                                              cplx_t<T>* table) {
+  const RtArgs<T>& a = tile.a;
+  ColsLayout<T, 1, 1, true> lay;
+  lay.tw_hi = a.tw_hi;
+  lay.tw_lo = a.tw_lo;
+  lay.split_shift = a.split_shift;
+  for (int q = threadIdx.x; q < R << a.line_shift; q += blockDim.x) {
+    lay.jmod = (unsigned)(tile.j0 + (q & (a.lines - 1))) % (unsigned)a.ns_outer;
+    T wr, wi;
+    lay.super_w((unsigned)((q >> a.line_shift) * bf), wr, wi);
+    st_global<T>(table + q, wr, wi);
+  }
+}
+template <typename T, int R>
+__device__ __forceinline__ void rt_super_apply(const RtTile<T, kRtColsTail>& tile,
+                                               const RtIo<T>& io, const cplx_t<T>* table,
+                                               T (&vr)[R], T (&vi)[R]) {
+  const RtArgs<T>& a = tile.a;
+  ColsLayout<T, 1, 1, true> lay;
+  lay.tw_hi = a.tw_hi;
+  lay.tw_lo = a.tw_lo;
+  lay.split_shift = a.split_shift;
+  lay.jmod = (unsigned)(tile.j0 + io.line) % (unsigned)a.ns_outer;
+  T br, bi;
+  lay.super_w((unsigned)io.j, br, bi);
+  cmul<T>(vr[0], vi[0], br, bi);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const cplx_t<T> v = ld_global<T>(io.gsrc + r * io.gsstep);
-        vr[r] = v.x;
-        vi[r] = v.y * io.sign;
+  for (int r = 1; r < R; ++r) {
+    const cplx_t<T> u = table[(r << a.line_shift) + io.line];
+    T xr = u.x, xi = u.y;
+    cmul<T>(xr, xi, br, bi);
+    cmul<T>(vr[r], vi[r], xr, xi);
+  }
+}
+
+// One stage: PER butterflies per thread (w = thread + m * threads).
+template <typename T, int MODE, int R, int PER, bool FIRST, bool LAST>
+__device__ __forceinline__ void rt_stage(const RtTile<T, MODE>& tile, const RtStage& s,
+                                         cplx_t<T>* sp) {
+  constexpr Where SRC = FIRST && MODE != kRtStaged ? kGlobal : kShared;
+  constexpr Where DST = LAST && (MODE == kRtRows || MODE == kRtColsTail) ? kGlobal : kShared;
+  constexpr bool SUPER = FIRST && MODE == kRtColsTail;
+  const RtArgs<T>& a = tile.a;
+  T vr[PER][R], vi[PER][R];
+#pragma unroll
+  for (int m = 0; m < PER; ++m) {
+    const RtIo<T> io = tile.template at<FIRST, LAST>(s, threadIdx.x + m * blockDim.x);
+    if (io.act) {
+      if constexpr (SRC == kGlobal) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const cplx_t<T> v = ld_global<T>(io.gsrc + r * io.gsstep);
+          vr[m][r] = v.x;
+          vi[m][r] = v.y * a.sign_in;
+        }
+      } else {
+        const cplx_t<T>* p = sp + io.src;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const cplx_t<T> v = p[r * io.sstep];
+          vr[m][r] = v.x;
+          vi[m][r] = v.y;
+        }
+      }
+      if constexpr (!SUPER) {
+        if constexpr (!FIRST) rt_twiddle<T, R>(vr[m], vi[m], io.tw, s.ns);
+        Dft<R>::fwd(vr[m], vi[m]);
       }
     } else {
-      const cplx_t<T>* p = sp + io.src;
+      // defined on every path: a register that is only written under `act` and
+      // read under it behind the barrier counts as live around the stage loop,
+      // for every radix at once (the radix-8 class spilled 350 bytes a thread)
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const cplx_t<T> v = p[r * io.sstep];
-        vr[r] = v.x;
-        vi[r] = v.y;
+      for (int r = 0; r < R; ++r) vr[m][r] = vi[m][r] = T(0);
+    }
+  }
+  if constexpr (SUPER) {
+    cplx_t<T>* table = sp + a.length * a.pitch;
+    rt_super_fill<T, R>(tile, s.bf, table);
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+      const RtIo<T> io = tile.template at<FIRST, LAST>(s, threadIdx.x + m * blockDim.x);
+      if (io.act) {
+        rt_super_apply<T, R>(tile, io, table, vr[m], vi[m]);
+        Dft<R>::fwd(vr[m], vi[m]);
       }
     }
-  } else {
-    // defined on every path: a register that is only written under `act` and
-    // read under it behind the barrier counts as live around the stage loop,
-    // for every radix at once (the radix-8 class spilled 350 bytes a thread)
-#pragma unroll
-    for (int r = 0; r < R; ++r) vr[r] = vi[r] = T(0);
-  }
-  if constexpr (Super::kActive) {
-    super.template fill<R>();
-    __syncthreads();
-  }
-  if (io.act) {
-    if constexpr (Super::kActive) super.template apply<R>(vr, vi);
-    if constexpr (TW) rt_twiddle<T, R>(vr, vi, io.tw, io.ns);
-    Dft<R>::fwd(vr, vi);
   }
   if constexpr (SRC == kShared && DST == kShared) __syncthreads();
-  if (io.act) {
-    if constexpr (DST == kGlobal) {
 #pragma unroll
-      for (int k = 0; k < R; ++k)
-        st_global<T>(io.gdst + k * io.gdstep, vr[k], vi[k] * io.sign);
-    } else {
-      cplx_t<T>* p = sp + io.dst;
+  for (int m = 0; m < PER; ++m) {
+    const RtIo<T> io = tile.template at<FIRST, LAST>(s, threadIdx.x + m * blockDim.x);
+    if (io.act) {
+      if constexpr (DST == kGlobal) {
 #pragma unroll
-      for (int k = 0; k < R; ++k) st_global<T>(p + k * io.dstep, vr[k], vi[k]);
+        for (int k = 0; k < R; ++k)
+          st_global<T>(io.gdst + k * io.gdstep, vr[m][k], vi[m][k] * a.sign_out);
+      } else {
+        cplx_t<T>* p = sp + io.dst;
+#pragma unroll
+        for (int k = 0; k < R; ++k) st_global<T>(p + k * io.dstep, vr[m][k], vi[m][k]);
+      }
     }
   }
   if constexpr (DST == kShared) __syncthreads();
 }
 
-struct RtNoSuper {
-  static constexpr bool kActive = false;
-};
+// Butterflies a thread may run in a radix-R stage of the several-butterfly
+// kernels (MULTI): as many as hold 16 points.
+__host__ __device__ constexpr int rt_per(int radix) { return radix > 8 ? 1 : 16 / radix; }
 
-// Super-stage twiddle of a later column pass: v[r] *= b u^r with b =
-// W^{jmod j} looked up by each thread and the powers u^r of the tile's lines
-// in a table (ColsLayout's scheme; here a line's jmod may wrap inside a tile).
-template <typename T>
-struct RtSuper {
-  static constexpr bool kActive = true;
-  ColsLayout<T, 1, 1, true> lay;   // the two-level table, this thread's jmod
-  cplx_t<T>* table;                // radix x lines
-  int j, bf, j0, line, line_shift;
-  unsigned ns;
-  template <int R>
-  __device__ __forceinline__ void fill() const {
-    ColsLayout<T, 1, 1, true> l = lay;
-    const int lines = 1 << line_shift;
-    for (int q = threadIdx.x; q < R << line_shift; q += blockDim.x) {
-      l.jmod = (unsigned)(j0 + (q & (lines - 1))) % ns;
-      T wr, wi;
-      l.super_w((unsigned)((q >> line_shift) * bf), wr, wi);
-      st_global<T>(table + q, wr, wi);
-    }
-  }
-  template <int R>
-  __device__ __forceinline__ void apply(T (&vr)[R], T (&vi)[R]) const {
-    T br, bi;
-    lay.super_w((unsigned)j, br, bi);
-    cmul<T>(vr[0], vi[0], br, bi);
-#pragma unroll
-    for (int r = 1; r < R; ++r) {
-      const cplx_t<T> u = table[(r << line_shift) + line];
-      T xr = u.x, xi = u.y;
-      cmul<T>(xr, xi, br, bi);
-      cmul<T>(vr[r], vi[r], xr, xi);
-    }
-  }
-};
-
-template <typename T, int MAXR, Where SRC, Where DST, bool TW, class Super>
-__device__ __forceinline__ void rt_dispatch(int radix, const RtIo<T>& io, cplx_t<T>* sp,
-                                            const Super& super) {
-#define MOFFT_RT_CASE(RR)                                                        \
-  case RR:                                                                       \
-    if constexpr (RR <= MAXR) rt_stage<T, RR, SRC, DST, TW>(io, sp, super);      \
+template <typename T, int MODE, int MAXR, bool MULTI, bool FIRST, bool LAST>
+__device__ __forceinline__ void rt_dispatch(const RtTile<T, MODE>& tile, const RtStage& s,
+                                            cplx_t<T>* sp) {
+#define MOFFT_RT_CASE(RR)                                                            \
+  case RR:                                                                           \
+    if constexpr (RR <= MAXR)                                                        \
+      rt_stage<T, MODE, RR, MULTI ? rt_per(RR) : 1, FIRST, LAST>(tile, s, sp);       \
     break;
-  switch (radix) {
+  switch (s.radix) {
     MOFFT_RT_CASE(2) MOFFT_RT_CASE(3) MOFFT_RT_CASE(4) MOFFT_RT_CASE(5)
     MOFFT_RT_CASE(6) MOFFT_RT_CASE(7) MOFFT_RT_CASE(8) MOFFT_RT_CASE(9)
     MOFFT_RT_CASE(10) MOFFT_RT_CASE(11) MOFFT_RT_CASE(12) MOFFT_RT_CASE(13)
@@ -238,146 +315,62 @@ __device__ __forceinline__ void rt_dispatch(int radix, const RtIo<T>& io, cplx_t
 #undef MOFFT_RT_CASE
 }
 
-template <typename T, int MODE, int MAXR, int MAXT>
+template <typename T, int MODE, int MAXR, bool MULTI, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) rt_kernel(const __grid_constant__ RtArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx_t<T>* sp = reinterpret_cast<cplx_t<T>*>(smem_raw);
   constexpr bool COLS = MODE >= kRtColsHead;
-  const cplx_t<T>* const in = after_previous(a.in);
+  RtTile<T, MODE> tile{a, after_previous(a.in), 0, 0, 0};
   const int tid = threadIdx.x;
   const int L = a.length;
   const int last = a.stage_count - 1;
-  long long b;
-  int j0 = 0, nl;
   if (COLS) {
     const unsigned groups = (unsigned)(a.total_lines + a.lines - 1) >> a.line_shift;
     const unsigned q = blockIdx.x / groups;
-    b = q;
-    j0 = (int)((blockIdx.x - q * groups) << a.line_shift);
-    nl = min(a.total_lines - j0, a.lines);
+    tile.b = q;
+    tile.j0 = (int)((blockIdx.x - q * groups) << a.line_shift);
+    tile.nl = min(a.total_lines - tile.j0, a.lines);
   } else {
-    b = (long long)blockIdx.x * a.lines;
-    nl = (int)(a.batch - b < a.lines ? a.batch - b : a.lines);
+    tile.b = (long long)blockIdx.x * a.lines;
+    tile.nl = (int)(a.batch - tile.b < a.lines ? a.batch - tile.b : a.lines);
   }
-  const int step = COLS ? a.pitch : 1;   // pairs between a line's points
-  // this thread's butterfly j of line `line` in a stage of bf butterflies
-  auto place = [&](const RtStage& s, int& line, int& j) {
-    if (COLS) {
-      line = tid & (a.lines - 1);
-      j = tid >> a.line_shift;
-      return j < s.bf && line < nl;
-    }
-    line = rt_div(tid, s.magic_bf);
-    j = tid - line * s.bf;
-    return line < nl;
-  };
-  auto middle = [&](const RtStage& s) {
-    RtIo<T> io;
-    int line, j;
-    io.act = place(s, line, j);
-    const int base = COLS ? line : line * a.pitch;
-    const int jq = rt_div(j, s.magic_ns), jm = j - jq * s.ns;
-    io.src = base + (j + jq * s.gpad) * step;
-    io.sstep = s.gstep * step;
-    io.dst = base + (jq * s.sblk + jm) * step;
-    io.dstep = s.ns * step;
-    io.tw = a.tw + s.twoff + jm;
-    io.ns = s.ns;
-    rt_dispatch<T, MAXR, kShared, kShared, true>(s.radix, io, sp, RtNoSuper());
-  };
-
-  // ---- first stage: Ns = 1
-  {
-    const RtStage& s = a.st[0];
-    RtIo<T> io;
-    int line, j;
-    io.act = place(s, line, j);
-    const int base = COLS ? line : line * a.pitch;
-    io.dst = base + j * s.sblk * step;
-    io.dstep = step;
-    io.sign = a.sign_in;
-    if constexpr (MODE == kRtStaged) {
-      // the tile's lines as they lie in global memory, kBatch loads in flight
-      constexpr int kBatch = sizeof(T) == 4 ? 8 : 4;
-      const int points = nl * L;
-      const cplx_t<T>* src = in + b * a.in_dist;
-      for (int q0 = tid; q0 < points; q0 += kBatch * blockDim.x) {
-        cplx_t<T> v[kBatch];
+  const long long b = tile.b;
+  const int points = tile.nl * L;
+  if constexpr (MODE == kRtStaged) {
+    // the tile's lines as they lie in global memory, kBatch loads in flight
+    constexpr int kBatch = sizeof(T) == 4 ? 8 : 4;
+    const cplx_t<T>* src = tile.in + b * a.in_dist;
+    for (int q0 = tid; q0 < points; q0 += kBatch * blockDim.x) {
+      cplx_t<T> v[kBatch];
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-          const int q = q0 + k * (int)blockDim.x;
-          const int ln = (int)__umulhi((unsigned)q, a.magic_len);
-          if (q < points) v[k] = ld_global<T>(src + ln * a.in_dist + (q - ln * L));
-        }
+      for (int k = 0; k < kBatch; ++k) {
+        const int q = q0 + k * (int)blockDim.x;
+        const int ln = (int)__umulhi((unsigned)q, a.magic_len);
+        if (q < points) v[k] = ld_global<T>(src + ln * a.in_dist + (q - ln * L));
+      }
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-          const int q = q0 + k * (int)blockDim.x;
-          const int ln = (int)__umulhi((unsigned)q, a.magic_len);
-          if (q < points) {
-            v[k].y *= a.sign_in;
-            sp[ln * a.pitch + (q - ln * L)] = v[k];
-          }
+      for (int k = 0; k < kBatch; ++k) {
+        const int q = q0 + k * (int)blockDim.x;
+        const int ln = (int)__umulhi((unsigned)q, a.magic_len);
+        if (q < points) {
+          v[k].y *= a.sign_in;
+          sp[ln * a.pitch + (q - ln * L)] = v[k];
         }
       }
-      __syncthreads();
-      io.src = base + j;
-      io.sstep = s.bf;
-      rt_dispatch<T, MAXR, kShared, kShared, false>(s.radix, io, sp, RtNoSuper());
-    } else if constexpr (MODE == kRtRows) {
-      io.gsrc = in + (b + line) * a.in_dist + j;
-      io.gsstep = s.bf;
-      rt_dispatch<T, MAXR, kGlobal, kShared, false>(s.radix, io, sp, RtNoSuper());
-    } else {
-      io.gsrc = in + b * a.in_dist + j0 + line + (long long)j * a.total_lines;
-      io.gsstep = (long long)a.total_lines * s.bf;
-      if constexpr (MODE == kRtColsHead) {
-        rt_dispatch<T, MAXR, kGlobal, kShared, false>(s.radix, io, sp, RtNoSuper());
-      } else {
-        RtSuper<T> super;
-        super.lay.tw_hi = a.tw_hi;
-        super.lay.tw_lo = a.tw_lo;
-        super.lay.split_shift = a.split_shift;
-        super.lay.jmod = (unsigned)(j0 + line) % (unsigned)a.ns_outer;
-        super.table = sp + L * a.pitch;
-        super.j = j;
-        super.bf = s.bf;
-        super.j0 = j0;
-        super.line = line;
-        super.line_shift = a.line_shift;
-        super.ns = (unsigned)a.ns_outer;
-        rt_dispatch<T, MAXR, kGlobal, kShared, false>(s.radix, io, sp, super);
-      }
     }
+    __syncthreads();
   }
   constexpr bool kStores = MODE == kRtRows || MODE == kRtColsTail;
+  rt_dispatch<T, MODE, MAXR, MULTI, true, false>(tile, a.st[0], sp);
   const int middles = kStores ? last : last + 1;
-  for (int i = 1; i < middles; ++i) middle(a.st[i]);
+  for (int i = 1; i < middles; ++i)
+    rt_dispatch<T, MODE, MAXR, MULTI, false, false>(tile, a.st[i], sp);
   if constexpr (kStores) {
-    // ---- last stage: Ns R = L, so j mod Ns = j
-    const RtStage& s = a.st[last];
-    RtIo<T> io;
-    int line, j;
-    io.act = place(s, line, j);
-    const int base = COLS ? line : line * a.pitch;
-    io.src = base + j * step;
-    io.sstep = s.gstep * step;
-    io.tw = a.tw + s.twoff + j;
-    io.ns = s.ns;
-    io.sign = a.sign_out;
-    if constexpr (MODE == kRtRows) {
-      io.gdst = a.out + (b + line) * a.out_dist + j;
-      io.gdstep = s.ns;
-    } else {
-      const unsigned ns = (unsigned)a.ns_outer, jl = (unsigned)(j0 + line), q = jl / ns;
-      io.gdst = a.out + b * a.out_dist + (long long)q * ns * L + (jl - q * ns) + j * a.ns_outer;
-      io.gdstep = a.ns_outer * s.ns;
-    }
-    rt_dispatch<T, MAXR, kShared, kGlobal, true>(s.radix, io, sp, RtNoSuper());
+    rt_dispatch<T, MODE, MAXR, MULTI, false, true>(tile, a.st[last], sp);
   } else {
     // kRtColsHead: lines j0 .. j0+nl-1 are one contiguous block of the
     // output; kRtStaged: the tile's lines leave as they arrived
-    const int points = nl * L;
-    cplx_t<T>* dst = COLS ? a.out + b * a.out_dist + (long long)j0 * L : a.out + b * a.out_dist;
+    cplx_t<T>* dst = a.out + b * a.out_dist + (COLS ? (long long)tile.j0 * L : 0);
     for (int q = tid; q < points; q += blockDim.x) {
       const int ln = (int)__umulhi((unsigned)q, a.magic_len);
       const int i = q - ln * L;

@@ -12,17 +12,30 @@ namespace mofft {
 // what the class needs unspilled (-Xptxas -v: FP32 37 / 48 / 63 registers for
 // radices up to 8 / 11 / 16, up to 80 in column passes with super-stage
 // twiddles; FP64 64 / 80 / 106, column passes 84 / 110 / 124).
-constexpr int rt_max_threads(int precision_bits, bool cols, int max_radix) {
+constexpr int rt_max_threads(int precision_bits, bool cols, int max_radix, bool multi) {
+  if (multi) return precision_bits == 32 ? (cols ? 768 : 1024) : 512;
   if (precision_bits == 32) return max_radix <= 11 || !cols ? 1024 : 768;
   if (max_radix <= 8) return cols ? 640 : 1024;
   if (max_radix <= 11) return cols ? 512 : 768;
   return 512;
 }
 
+// Registers per thread of those kernels as compiled (the larger of the first
+// and later column passes), for the planner's occupancy.
+constexpr int rt_registers(int precision_bits, bool cols, int max_radix, bool multi) {
+  if (precision_bits == 32) {
+    if (multi) return cols ? 80 : 64;
+    return max_radix <= 8 ? (cols ? 48 : 40) : max_radix <= 11 ? (cols ? 64 : 48) : cols ? 80 : 56;
+  }
+  if (multi) return cols ? 128 : 112;
+  return max_radix <= 8 ? (cols ? 72 : 64) : max_radix <= 11 ? (cols ? 88 : 80) : cols ? 128 : 104;
+}
+
 struct RtShape {
   int lines;       // lines per CTA
   int threads;     // CTA threads: the most butterflies of any stage, whole warps
   int max_radix;   // largest radix of the chain
+  int multi;       // several butterflies per thread (rt_per)
   int pitch;       // pairs per line (ROWS) / per element row (COLS)
   int staged;      // ROWS: global I/O goes through the tile
   int pad[16];     // pad pairs behind each block of the exchange after stage i

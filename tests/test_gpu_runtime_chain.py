@@ -25,6 +25,9 @@ CASES = [
     (2197, None, 5), (2744, [14, 14, 14], 2), (4095, None, 3), (5005, None, 2), (6561, None, 2),
     (9009, None, 1), (12005, None, 1),
     (4096, [2] * 12, 2),              # more butterflies than a CTA has threads
+    # several butterflies per thread: uneven radices, small ones, the limits
+    (35, None, 300), (243, None, 7), (500, None, 5), (2500, [10, 10, 5, 5], 3), (3125, None, 2),
+    (4000, None, 3), (7007, None, 1), (12740, None, 2), (390625, None, 1),
     (28561, None, 3), (50625, None, 2), (30030, None, 1), (117649, None, 1), (531441, None, 1),
 ]
 
