@@ -111,7 +111,7 @@ __device__ __forceinline__ void rt_twiddle(T (&vr)[R], T (&vi)[R],
 // computes only the addresses it uses.
 enum RtMode {
   kRtRows = 0,      // whole transforms, first and last stage on global memory
-  kRtStaged = 1,    // whole transforms copied through the tile
+  kRtStaged = 1,    // whole transforms of one stage, copied through the tile
   kRtColsHead = 2,  // first pass of a multi-pass transform (Ns = 1)
   kRtColsTail = 3   // later pass: super-stage twiddles, strided stores
 };

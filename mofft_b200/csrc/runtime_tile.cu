@@ -97,11 +97,11 @@ static bool rt_form(int precision_bits, bool cols, bool multi, int length, const
   s.smem = (size_t)lines * s.pitch * cb;
   if (s.smem > kSmemLimit) return false;
   s.threads = (threads(lines) + 31) / 32 * 32;
-  // runs of the direct loads (L / first radix) and stores (L / last radix)
-  // under 64 bytes: copy the lines through the tile instead (FP32 n = 144,
-  // runs of 96 bytes: 174 us through the tile, 90 direct)
-  const int in_run = length / chain[0], out_run = length / chain[count - 1];
-  s.staged = count < 2 || in_run < row / 2 || out_run < row / 2;
+  // one stage: its only butterfly reads and writes whole short lines, so the
+  // lines are copied through the tile.  More stages run direct however short
+  // their runs (FP32 50 = 10 5 170 us through the tile, 111 direct; 25 157 and
+  // 118; 144 174 and 90; FP64 26 = 13 2 298 and 120)
+  s.staged = count < 2;
   *out = s;
   return true;
 }
@@ -113,15 +113,18 @@ static bool rt_form(int precision_bits, bool cols, bool multi, int length, const
 // then idle (FP32 4000 = 10 10 8 5 271 -> 186 us, 500 = 10 10 5 156 -> 120;
 // FP64 2500 = 10 10 5 5 236 -> 158) or small radices for most of a CTA's
 // (FP32 3125 = 5^5 236 -> 206; column passes of 625 points 656 -> 511).
-// Lines copied through the tile: several for FP32 with a radix up to 5
-// (21 = 7 3 199 -> 154, 20 = 5 4 162 -> 136), never for FP64 (21 146 -> 194).
-static bool several_butterflies(int precision_bits, bool cols, const int *chain, int count,
-                                const RtShape &one) {
+static bool several_butterflies(int precision_bits, bool cols, int length, const int *chain,
+                                int count, const RtShape &one) {
   int least = 64;
   for (int i = 0; i < count; ++i)
     if (chain[i] < least) least = chain[i];
   if (cols) return one.threads > 640;
-  if (one.staged) return precision_bits == 32 && least <= 5;
+  if (one.staged) return false;
+  // short FP32 lines of unequal radices up to 8: a butterfly is too little work for a
+  // thread of its own (20 = 5 4 195 -> 114, 28 = 7 4 209 -> 109)
+  if (precision_bits == 32 && length < 64 && least <= 5 && one.max_radix > least &&
+      one.max_radix <= 8)
+    return true;
   return one.max_radix >= 2 * least || (least <= 5 && one.threads > 512);
 }
 
@@ -133,7 +136,7 @@ bool rt_shape(int precision_bits, bool cols, int length, const int *chain, int c
   RtShape several;
   const bool one = rt_form(precision_bits, cols, false, length, chain, count, units, line_units,
                            out);
-  if (one && !several_butterflies(precision_bits, cols, chain, count, *out)) return true;
+  if (one && !several_butterflies(precision_bits, cols, length, chain, count, *out)) return true;
   if (!rt_form(precision_bits, cols, true, length, chain, count, units, line_units, &several))
     return one;
   *out = several;
