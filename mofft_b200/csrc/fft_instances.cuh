@@ -336,6 +336,7 @@ const Entry *entries_cols_f32(int *count);
 const Entry *entries_cols_f64(int *count);
 const Entry *entries_rows_mixed(int *count);
 const Entry *entries_rows_even(int *count);
+const Entry *entries_twin_f32(int *count);
 const Entry *entries_cols_mixed(int *count);
 const Entry *entries_tensor(int *count);
 const Entry *entries_tensor64(int *count);

@@ -18,7 +18,7 @@ const std::vector<Entry> &registry() {
                                       entries_rows_f32,
                                       entries_rows_f64, entries_cols_f32,
                                       entries_cols_f64, entries_rows_mixed,
-                                      entries_rows_even,
+                                      entries_rows_even, entries_twin_f32,
                                       entries_cols_mixed, entries_tensor64,
                                       entries_tensor, entries_cluster};
     for (auto list : lists) {

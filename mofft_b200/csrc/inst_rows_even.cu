@@ -50,7 +50,6 @@ const Entry *entries_rows_even(int *count) {
       ROWSDP(double, 64, 8, 16, 8, 8),
       ROWSDP(double, 48, 8, 16, 6, 8),
       ROWSDP(double, 32, 4, 32, 8, 4),
-      ROWSDP(double, 16, 4, 64, 4, 4),
       ROWSDP(double, 640, 80, 2, 8, 8, 10),
       ROWSDP(float, 768, 64, 2, 16, 12, 4),
   };

@@ -1,0 +1,295 @@
+// Twin one-pass kernels: every thread transforms two lines at once with packed
+// FP32 arithmetic.
+//
+// The one-pass FP32 kernels issue 65 instructions a point (n = 4096, 71 % of
+// the issue slots at full clock) and become issue-bound when the clock falls
+// under load.  sm_100 executes add, sub, mul and fma on pairs of FP32 values
+// (.f32x2) in one instruction.  Two transforms b, b+1 need the same operations
+// on the same butterfly, so a thread keeps the real parts of both in one
+// register pair and the imaginary parts in another: the codelets, twiddle
+// products and exchanges, and all index arithmetic, are issued once for two
+// lines.  A value pair crosses shared memory as one 16-byte access
+// {reA, reB, imA, imB}, the layout of the FP64 pair tiles.
+//
+// Measured against the one-line instances (us, 2^26 points / 2^21 points in
+// L2): 64 164 -> 154 / 8.1 -> 7.9, 128 177 -> 162 / 10.0 -> 8.9, 256 158 -> 157
+// / 9.4 -> 7.7, 320 209 -> 177, 384 184 -> 156, 512 169 -> 156 / 9.1 -> 8.8,
+// 1280 183 -> 169, 1536 168 -> 160; under sustained load 256 174 -> 164, 512
+// 196 -> 182.  Not built where one line already takes half an SM's tile or
+// registers: a pair halves the resident CTAs, whose barriers then show (4096
+// 170 -> 181, 8192 223 -> 291, 3072 171 -> 189, 2560 177 -> 205), nor where it
+// loses in L2 (160, 192, 640, 768, 1024, 2048).
+#pragma once
+
+#include "fft_device.cuh"
+
+namespace mofft {
+
+// Two FP32 values.  `neg` and `cst` are compile-time knowledge (every use is
+// inlined and unrolled): a negation only flips `neg`, which the next add or sub
+// absorbs, and a constant factor changes its sign for free.
+struct TwinProd;
+struct Twin {
+  unsigned long long v;
+  float c;         // value of a constant
+  bool neg, cst;
+  __device__ __forceinline__ Twin() : v(0), c(0.f), neg(false), cst(false) {}
+  __device__ __forceinline__ explicit Twin(unsigned long long raw)
+      : v(raw), c(0.f), neg(false), cst(false) {}
+  __device__ __forceinline__ explicit Twin(double x)
+      : v(0), c((float)x), neg(false), cst(true) {}
+  __device__ __forceinline__ explicit Twin(int x)
+      : v(0), c((float)x), neg(false), cst(true) {}
+  __device__ __forceinline__ Twin(const TwinProd& p);
+};
+
+__device__ __forceinline__ unsigned long long twin_pack(float a, float b) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+__device__ __forceinline__ void twin_unpack(unsigned long long v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long twin_add(unsigned long long a,
+                                                       unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long twin_sub(unsigned long long a,
+                                                       unsigned long long b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long twin_mul(unsigned long long a,
+                                                       unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long twin_fma(unsigned long long a,
+                                                       unsigned long long b,
+                                                       unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// The value itself: constants as a pair, a pending negation applied.
+__device__ __forceinline__ unsigned long long twin_value(const Twin& a) {
+  if (a.cst) return twin_pack(a.neg ? -a.c : a.c, a.neg ? -a.c : a.c);
+  if (a.neg) return a.v ^ 0x8000000080000000ull;
+  return a.v;
+}
+// Without its sign (for operations that take the sign elsewhere).
+__device__ __forceinline__ unsigned long long twin_plain(const Twin& a) {
+  return a.cst ? twin_pack(a.c, a.c) : a.v;
+}
+__device__ __forceinline__ Twin twin_signed(unsigned long long v, bool neg) {
+  Twin r(v);
+  r.neg = neg;
+  return r;
+}
+
+// A product not yet added to anything.
+struct TwinProd {
+  Twin a, b;
+};
+__device__ __forceinline__ TwinProd operator*(const Twin& a, const Twin& b) {
+  TwinProd p;
+  p.a = a;
+  p.b = b;
+  return p;
+}
+__device__ __forceinline__ Twin twin_of(const TwinProd& p) {
+  return twin_signed(twin_mul(twin_plain(p.a), twin_plain(p.b)), p.a.neg != p.b.neg);
+}
+__device__ __forceinline__ Twin operator-(const Twin& a) {
+  Twin r = a;
+  r.neg = !a.neg;
+  return r;
+}
+__device__ __forceinline__ TwinProd operator-(const TwinProd& p) {
+  TwinProd r = p;
+  r.a.neg = !p.a.neg;
+  return r;
+}
+__device__ __forceinline__ Twin operator+(const Twin& a) { return a; }
+__device__ __forceinline__ Twin operator+(const Twin& a, const Twin& b) {
+  if (a.neg == b.neg) return twin_signed(twin_add(twin_plain(a), twin_plain(b)), a.neg);
+  if (b.neg) return twin_signed(twin_sub(twin_plain(a), twin_plain(b)), false);
+  return twin_signed(twin_sub(twin_plain(b), twin_plain(a)), false);
+}
+__device__ __forceinline__ Twin operator-(const Twin& a, const Twin& b) { return a + (-b); }
+__device__ __forceinline__ Twin::Twin(const TwinProd& p) { *this = twin_of(p); }
+// a + p: the product's sign relative to a goes into a constant factor; two
+// variable factors of the other sign multiply first.
+__device__ __forceinline__ Twin operator+(const Twin& a, const TwinProd& p) {
+  const bool flip = (p.a.neg != p.b.neg) != a.neg;
+  if (!flip)
+    return twin_signed(twin_fma(twin_plain(p.a), twin_plain(p.b), twin_plain(a)), a.neg);
+  if (p.b.cst)
+    return twin_signed(twin_fma(twin_plain(p.a), twin_pack(-p.b.c, -p.b.c), twin_plain(a)),
+                       a.neg);
+  if (p.a.cst)
+    return twin_signed(twin_fma(twin_pack(-p.a.c, -p.a.c), twin_plain(p.b), twin_plain(a)),
+                       a.neg);
+  return a + twin_of(p);
+}
+__device__ __forceinline__ Twin operator+(const TwinProd& p, const Twin& a) { return a + p; }
+__device__ __forceinline__ Twin operator-(const Twin& a, const TwinProd& p) { return a + (-p); }
+__device__ __forceinline__ Twin operator-(const TwinProd& p, const Twin& a) { return (-a) + p; }
+__device__ __forceinline__ Twin operator+(const TwinProd& p, const TwinProd& q) {
+  return twin_of(p) + q;
+}
+__device__ __forceinline__ Twin operator-(const TwinProd& p, const TwinProd& q) {
+  return twin_of(p) + (-q);
+}
+
+// Where a thread's two lines lie.
+struct TwinLines {
+  const float2* ga;
+  const float2* gb;
+  float2* oa;
+  float2* ob;
+  bool active, both;          // line A / both lines inside the batch
+  ulonglong2* sp;             // the pair's shared tile
+  unsigned long long sign;    // {1, 1} or {-1, -1}: conjugation on load and store
+};
+
+// x *= w with one scalar twiddle for both lines.
+__device__ __forceinline__ void twin_rotate(Twin& xr, Twin& xi, float wr, float wi) {
+  const Twin cr(twin_pack(wr, wr)), ci(twin_pack(wi, wi));
+  const Twin r = xr * cr - xi * ci;
+  const Twin i = xi * cr + xr * ci;
+  xr = r;
+  xi = i;
+}
+
+// Stage twiddles v[r] *= w^r.  Radix 16: w^1 .. w^4, w^8, w^12 from the table,
+// the others one product (computed once for both lines).
+template <int R, int NS>
+__device__ __forceinline__ void twin_twiddle(Twin (&vr)[R], Twin (&vi)[R],
+                                             const float2* __restrict__ tw) {
+  float2 low[4];
+#pragma unroll
+  for (int k = 1; k < 4; ++k)
+    if (k < R) low[k] = __ldg(tw + (k - 1) * NS);
+#pragma unroll
+  for (int q = 0; q < R; q += 4) {
+    float2 base;
+    if (q > 0) {
+      base = __ldg(tw + (q - 1) * NS);
+      twin_rotate(vr[q], vi[q], base.x, base.y);
+    }
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {
+      if (q + k < R) {
+        float wr = low[k].x, wi = low[k].y;
+        if (q > 0) cmul<float>(wr, wi, base.x, base.y);
+        twin_rotate(vr[q + k], vi[q + k], wr, wi);
+      }
+    }
+  }
+}
+
+template <int L, int TPL, int SH, int NS, int TWOFF, int R, int... Rest>
+struct TwinRunner {
+  static constexpr int BF = L / R;
+  static constexpr int PER = (BF + TPL - 1) / TPL;
+  static constexpr bool EVEN = BF % TPL == 0;
+  static constexpr bool FIRST = NS == 1;
+  static constexpr bool LAST = sizeof...(Rest) == 0;
+  __device__ __forceinline__ static int pad(int i) { return SH ? i + (i >> SH) : i; }
+  __device__ __forceinline__ static void run(const TwinLines& t, int tid,
+                                             const float2* __restrict__ tw) {
+    Twin vr[PER][R], vi[PER][R];
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+      const int j = tid + m * TPL;
+      if (EVEN || j < BF) {
+        if constexpr (FIRST) {
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const int i = j + r * BF;
+            float2 a = make_float2(0.f, 0.f), b = a;
+            if (t.active) a = ld_global<float>(t.ga + i);
+            if (t.both) b = ld_global<float>(t.gb + i);
+            vr[m][r] = Twin(twin_pack(a.x, b.x));
+            vi[m][r] = Twin(twin_mul(twin_pack(a.y, b.y), t.sign));
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const ulonglong2 v = t.sp[pad(j + r * BF)];
+            vr[m][r] = Twin(v.x);
+            vi[m][r] = Twin(v.y);
+          }
+          twin_twiddle<R, NS>(vr[m], vi[m], tw + TWOFF + j % NS);
+        }
+        Dft<R>::fwd(vr[m], vi[m]);
+      }
+    }
+    if constexpr (!FIRST && !LAST) __syncthreads();
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+      const int j = tid + m * TPL;
+      if (EVEN || j < BF) {
+        const int base = (j / NS) * NS * R + (j % NS);
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+          const int i = base + k * NS;
+          if constexpr (LAST) {
+            float ra, rb, ia, ib;
+            twin_unpack(twin_value(vr[m][k]), ra, rb);
+            twin_unpack(twin_mul(twin_value(vi[m][k]), t.sign), ia, ib);
+            if (t.active) st_global<float>(t.oa + i, ra, ia);
+            if (t.both) st_global<float>(t.ob + i, rb, ib);
+          } else {
+            t.sp[pad(i)] = make_ulonglong2(twin_value(vr[m][k]), twin_value(vi[m][k]));
+          }
+        }
+      }
+    }
+    if constexpr (!LAST) {
+      __syncthreads();
+      TwinRunner<L, TPL, SH, NS * R, TWOFF + stage_table_size(R, NS), Rest...>::run(t, tid, tw);
+    }
+  }
+};
+
+// TP line pairs per CTA, TPL threads per pair.
+template <int L, int TPL, int TP, int SH>
+struct TwinGeom {
+  static constexpr int THREADS = TPL * TP;
+  static constexpr int PITCH = pair_pitch<double>(L, TPL, TP, SH);
+  static constexpr size_t SMEM = (size_t)TP * PITCH * 16;
+  // 128 registers: 16 points of two lines take 64
+  static constexpr int MIN_RAW = 65536 / (128 * ((THREADS + 31) / 32 * 32));
+  static constexpr int MIN_CTAS = MIN_RAW < 1 ? 1 : MIN_RAW;
+};
+
+template <int L, int TPL, int TP, int SH, int... Rs>
+__global__ void __launch_bounds__(TPL * TP, (TwinGeom<L, TPL, TP, SH>::MIN_CTAS))
+twin_kernel(const RowsArgs<float> args) {
+  static_assert(StageProduct<L, Rs...>::value == L, "radices must multiply to L");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RowsArgs<float> a = args;
+  a.in = after_previous(args.in);
+  const int pair = threadIdx.x / TPL;
+  const long long b = 2 * ((long long)blockIdx.x * TP + pair);
+  TwinLines t;
+  t.active = b < a.batch;
+  t.both = b + 1 < a.batch;
+  t.ga = t.active ? batch_in<float>(a.in, a.in_dist, a.in_table, b) : a.in;
+  t.gb = t.both ? batch_in<float>(a.in, a.in_dist, a.in_table, b + 1) : t.ga;
+  t.oa = t.active ? batch_out<float>(a.out, a.out_dist, a.out_table, b) : a.out;
+  t.ob = t.both ? batch_out<float>(a.out, a.out_dist, a.out_table, b + 1) : t.oa;
+  t.sp = reinterpret_cast<ulonglong2*>(smem_raw) + pair * TwinGeom<L, TPL, TP, SH>::PITCH;
+  t.sign = twin_pack(a.sign, a.sign);
+  TwinRunner<L, TPL, SH, 1, 0, Rs...>::run(t, threadIdx.x % TPL, a.tw);
+}
+
+}  // namespace mofft
