@@ -262,7 +262,8 @@ struct ColsLayout {
   // shared memory.  (Every thread looking up u .. u^3, u^4, u^8, u^12 for
   // itself: 14 loads and the index arithmetic of seven table entries per
   // butterfly, 13 instructions a point; the second pass of FP32 65536 took
-  // 109 us of 2^25 points where the first, without twiddles, took 85.)
+  // 109 us of 2^25 points where the first, without twiddles, took 85; the
+  // shared table brings it to 100.)
   template <int R, int BF, int THREADS>
   __device__ __forceinline__ void super_fill() const {
     ColsLayout l = *this;

@@ -17,6 +17,8 @@
 // 134 -> 96, 640 103 -> 91, 1280 105 -> 95, 3072 101 -> 90; FP64 48 105 -> 81,
 // 64 96 -> 82, 128 93 -> 81, 192 107 -> 84, 320 132 -> 90, 384 120 -> 87, 640
 // 100 -> 89, 1280 119 -> 93, 2048 99 -> 88, 6144 168 -> 156.
+// Tuned FP32 plans of 64, 320, 384, 1280 and 1536 points have moved on to the
+// two-line kernels of twin_fft.cuh (77, 89, 78, 85 and 80 us).
 #include "fft_instances.cuh"
 
 namespace mofft {

@@ -292,4 +292,227 @@ twin_kernel(const RowsArgs<float> args) {
   TwinRunner<L, TPL, SH, 1, 0, Rs...>::run(t, threadIdx.x % TPL, a.tw);
 }
 
+// ---------------------------------------------------------------------------
+// Twin column passes: a thread runs the same butterfly of two adjacent lines
+// (2 pr, 2 pr + 1) of the tile.  Their elements are adjacent in global memory,
+// so one 16-byte access moves both where the transform starts on a 16-byte
+// boundary (8-byte accesses where it does not), and in the tile one 16-byte
+// word {reA, reB, imA, imB}.  Stage twiddles are the same for both lines; the
+// line powers of a later pass (ColsLayout::super_fill) are kept as packed pairs.
+//
+// Lines of 320-512 points are bound by their tiles: 8 lines on 256 threads move
+// 64-byte runs, and 16 lines of the one-line form take 512 threads at 64
+// registers.  Two lines a thread give 16 lines, 128-byte runs, on 256 threads
+// at 110 registers with two CTAs per SM.  us per 2^25 points, 8 lines -> 16
+// lines one a thread -> 16 lines two a thread: 512 x 160 224 -> 211 -> 199, 512
+// x 192 220 -> 206 -> 194, 256 x 512 209 -> 209 -> 199, 512 x 1024 261 -> 248
+// -> 237; 512 x 512 239 -> 218 (256 x 1024 takes 220); as the narrow side of
+// 327680 and 393216, 320 and 384 points take
+// 279 -> 252 and 260 -> 247.  In L2 (2^21 points) 98304 18.6 -> 15.7, 131072
+// 17.6 -> 15.6.  One transform alone, with half the CTAs, takes up to 1.2 us
+// longer (131072 7.8 -> 9.0).  Not built for 64-256 points, whose one-line
+// tiles already move 128-byte runs (256 x 256 184 -> 187, 64 x 64 170 -> 168),
+// nor for 640-2048 points, whose 16-line tiles leave one CTA per SM (512 x
+// 1024 237 -> 245).
+// ---------------------------------------------------------------------------
+template <int L, int TPL, int C>
+struct TwinColsGeom {
+  static constexpr int P = C / 2;                 // line pairs
+  static constexpr int THREADS = TPL * P;
+  static constexpr int PITCH = P + 1;             // 16-byte words per element row
+  static constexpr size_t SMEM = (size_t)L * PITCH * 16;
+  static constexpr size_t super_smem(int first_radix) {
+    return SMEM + (size_t)first_radix * P * 16;
+  }
+  static constexpr int MIN_RAW = 65536 / (128 * ((THREADS + 31) / 32 * 32));
+  static constexpr int MIN_CTAS = MIN_RAW < 1 ? 1 : MIN_RAW;
+};
+
+template <int L, int TPL, int C, bool HEAD>
+struct TwinCols {
+  using G = TwinColsGeom<L, TPL, C>;
+  const ColsArgs<float>& a;
+  const float2* gin;          // element 0 of line 2 pr
+  float2* gout;
+  long long in_stride, out_stride;
+  bool in16, out16;           // 16-byte aligned pairs
+  ulonglong2* sp;             // the tile
+  ulonglong2* sw;             // line powers (later passes)
+  unsigned jmod;              // of line 2 pr
+  int pr;
+  unsigned long long sign_in, sign_out;
+
+  // W^{jm i} of one line from the two-level table
+  __device__ __forceinline__ float2 power(unsigned jm, unsigned i) const {
+    ColsLayout<float, 1, 1, true> lay;
+    lay.tw_hi = a.tw_hi;
+    lay.tw_lo = a.tw_lo;
+    lay.split_shift = a.split_shift;
+    lay.jmod = jm;
+    float2 w;
+    lay.super_w(i, w.x, w.y);
+    return w;
+  }
+
+  template <int NS, int TWOFF, int R, int... Rest>
+  __device__ __forceinline__ void run(int t, const float2* __restrict__ tw) const {
+    constexpr int BF = L / R;
+    constexpr int PER = (BF + TPL - 1) / TPL;
+    constexpr bool EVEN = BF % TPL == 0;
+    constexpr bool FIRST = NS == 1;
+    constexpr bool LAST = sizeof...(Rest) == 0;
+    constexpr bool STORE = LAST && !HEAD;
+    Twin vr[PER][R], vi[PER][R];
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+      const int j = t + m * TPL;
+      if (EVEN || j < BF) {
+        if constexpr (FIRST) {
+          const float2* p = gin + (long long)j * in_stride;
+          const long long step = (long long)BF * in_stride;
+          if (in16) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
+              vr[m][r] = Twin(twin_pack(v.x, v.z));
+              vi[m][r] = Twin(twin_mul(twin_pack(v.y, v.w), sign_in));
+              p += step;
+            }
+          } else {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const float2 x = ld_global<float>(p), y = ld_global<float>(p + 1);
+              vr[m][r] = Twin(twin_pack(x.x, y.x));
+              vi[m][r] = Twin(twin_mul(twin_pack(x.y, y.y), sign_in));
+              p += step;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const ulonglong2 v = sp[(j + r * BF) * G::PITCH + pr];
+            vr[m][r] = Twin(v.x);
+            vi[m][r] = Twin(v.y);
+          }
+        }
+      }
+    }
+    if constexpr (FIRST && !HEAD) {
+      // the tile's line powers u^r, filled while the loads are in flight
+      for (int q = threadIdx.x; q < R * G::P; q += G::THREADS) {
+        const unsigned jm = jmod - 2u * (unsigned)pr + 2u * (unsigned)(q % G::P);
+        const unsigned i = (unsigned)(q / G::P * BF);
+        const float2 x = power(jm, i), y = power(jm + 1, i);
+        sw[q] = make_ulonglong2(twin_pack(x.x, y.x), twin_pack(x.y, y.y));
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+      const int j = t + m * TPL;
+      if (EVEN || j < BF) {
+        if constexpr (FIRST && !HEAD) {
+          const float2 x = power(jmod, (unsigned)j), y = power(jmod + 1, (unsigned)j);
+          const Twin br(twin_pack(x.x, y.x)), bi(twin_pack(x.y, y.y));
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            Twin wr = br, wi = bi;
+            if (r > 0) {
+              const ulonglong2 u = sw[r * G::P + pr];
+              const Twin ur(u.x), ui(u.y);
+              wr = ur * br - ui * bi;
+              wi = ui * br + ur * bi;
+            }
+            const Twin xr = vr[m][r] * wr - vi[m][r] * wi;
+            const Twin xi = vi[m][r] * wr + vr[m][r] * wi;
+            vr[m][r] = xr;
+            vi[m][r] = xi;
+          }
+        }
+        if constexpr (!FIRST) twin_twiddle<R, NS>(vr[m], vi[m], tw + TWOFF + j % NS);
+        Dft<R>::fwd(vr[m], vi[m]);
+      }
+    }
+    if constexpr (!FIRST && !STORE) __syncthreads();
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+      const int j = t + m * TPL;
+      if (EVEN || j < BF) {
+        const int base = (j / NS) * NS * R + (j % NS);
+        if constexpr (STORE) {
+          float2* p = gout + (long long)base * out_stride;
+          const long long step = (long long)NS * out_stride;
+#pragma unroll
+          for (int k = 0; k < R; ++k) {
+            float ra, rb, ia, ib;
+            twin_unpack(twin_value(vr[m][k]), ra, rb);
+            twin_unpack(twin_mul(twin_value(vi[m][k]), sign_out), ia, ib);
+            if (out16) {
+              *reinterpret_cast<float4*>(p) = make_float4(ra, ia, rb, ib);
+            } else {
+              st_global<float>(p, ra, ia);
+              st_global<float>(p + 1, rb, ib);
+            }
+            p += step;
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < R; ++k)
+            sp[(base + k * NS) * G::PITCH + pr] =
+                make_ulonglong2(twin_value(vr[m][k]), twin_value(vi[m][k]));
+        }
+      }
+    }
+    if constexpr (!STORE) __syncthreads();
+    if constexpr (!LAST) run<NS * R, TWOFF + stage_table_size(R, NS), Rest...>(t, tw);
+  }
+};
+
+template <int L, int TPL, int C, bool HEAD, int... Rs>
+__global__ void __launch_bounds__(TPL * C / 2, (TwinColsGeom<L, TPL, C>::MIN_CTAS))
+twin_cols_kernel(const ColsArgs<float> args) {
+  static_assert(StageProduct<L, Rs...>::value == L, "radices must multiply to L");
+  static_assert(C % 2 == 0, "lines in pairs");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  using G = TwinColsGeom<L, TPL, C>;
+  ColsArgs<float> a = args;
+  a.in = after_previous(args.in);
+  long long b, j0;
+  cols_tile<L, C>(a, b, j0);
+  const int pr = threadIdx.x % G::P;
+  const unsigned ns = (unsigned)a.ns_outer;             // a multiple of C, or 1
+  const unsigned j = (unsigned)j0 + 2u * (unsigned)pr;
+  const unsigned jq = HEAD ? 0u : j / ns, jm = j - jq * ns;
+  const float2* in_b = batch_in<float>(a.in, a.in_dist, a.in_table, b);
+  float2* out_b = batch_out<float>(a.out, a.out_dist, a.out_table, b);
+  const long long stride = a.total / L;                 // a multiple of C
+  TwinCols<L, TPL, C, HEAD> tc{a,
+                               in_b + j,
+                               out_b + (long long)jq * ns * L + jm,
+                               stride,
+                               (long long)ns,
+                               (reinterpret_cast<uintptr_t>(in_b) & 15) == 0,
+                               (reinterpret_cast<uintptr_t>(out_b) & 15) == 0,
+                               reinterpret_cast<ulonglong2*>(smem_raw),
+                               reinterpret_cast<ulonglong2*>(smem_raw + G::SMEM),
+                               jm,
+                               pr,
+                               twin_pack(a.sign_in, a.sign_in),
+                               twin_pack(a.sign_out, a.sign_out)};
+  tc.template run<1, 0, Rs...>(threadIdx.x / G::P, a.tw);
+  if constexpr (HEAD) {
+    // lines j0 .. j0+C-1 are one contiguous block of the output
+    float2* dst = out_b + j0 * L;
+    for (int q = threadIdx.x; q < G::P * L; q += G::THREADS) {
+      const int p = q / L, k = q - p * L;
+      const ulonglong2 v = tc.sp[k * G::PITCH + p];
+      float ra, rb, ia, ib;
+      twin_unpack(v.x, ra, rb);
+      twin_unpack(twin_mul(v.y, tc.sign_out), ia, ib);
+      st_global<float>(dst + (2 * p) * L + k, ra, ia);
+      st_global<float>(dst + (2 * p + 1) * L + k, rb, ib);
+    }
+  }
+}
+
 }  // namespace mofft
