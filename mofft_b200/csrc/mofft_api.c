@@ -1313,11 +1313,14 @@ static mofft_status ensure_staging(mofft_core *c, size_t chunks) {
 /* Largest span of a host-buffer execute that runs on mapped pinned memory.
  * The kernel then reads and writes the host's memory itself, so a call is two
  * host copies and one launch: 1024 FP32 points in 19 us instead of 26 with two
- * pageable transfers around the launch, 16384 points in 34 instead of 54.
+ * pageable transfers around the launch, 16384 points in 34 instead of 54, 256
+ * KiB in 51 instead of 73.  Beyond that the host's own copies take most of a
+ * call and the gain shrinks to the spread between hosts (400 to 500 KiB: 91 to
+ * 114 us on both paths, one host 25 % slower on this one).
  * Allocating that memory takes 1.3 to 3 ms, some hundred times the saving: a
  * plan does it at its 32nd such call, so plans that run a few times never pay
  * it. */
-#define MOFFT_PINNED_SPAN ((size_t)512 << 10)
+#define MOFFT_PINNED_SPAN ((size_t)256 << 10)
 #define MOFFT_PINNED_CALLS 32u
 
 /* One-pass schedules without bulk copies of their input (those kernels also
