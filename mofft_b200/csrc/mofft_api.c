@@ -1360,6 +1360,26 @@ static mofft_status execute_pinned(mofft_core *c, const void *in, void *out, siz
   return MOFFT_SUCCESS;
 }
 
+/* `count` staged transforms to the host: the gaps between strided transforms
+ * belong to the caller and stay as they are.  A gap past the pitch that the
+ * strided copy takes (2^31 - 1 bytes) needs a copy per transform. */
+static cudaError_t download(const mofft_core *c, void *out, const void *dout, size_t count,
+                            cudaStream_t stream) {
+  const size_t cb = mofft_complex_bytes(c->precision_bits);
+  const size_t line = c->length * cb, pitch = c->distance * cb;
+  if (line == pitch || count == 1)
+    return cudaMemcpyAsync(out, dout, count * line, cudaMemcpyDeviceToHost, stream);
+  if (pitch <= 0x7fffffffu)
+    return cudaMemcpy2DAsync(out, pitch, dout, pitch, line, count, cudaMemcpyDeviceToHost,
+                             stream);
+  cudaError_t err = cudaSuccess;
+  for (size_t b = 0; b < count && err == cudaSuccess; ++b)
+    err = cudaMemcpyAsync((unsigned char *)out + b * pitch,
+                          (const unsigned char *)dout + b * pitch, line,
+                          cudaMemcpyDeviceToHost, stream);
+  return err;
+}
+
 /* Host buffers (pageable or pinned), c->lock held: staged through plan-owned
  * memory.  Chunks of about 24 MiB flow through three streams: uploads in order
  * on one, each chunk's passes on another once its upload has landed, downloads
@@ -1400,8 +1420,7 @@ static mofft_status execute_host(mofft_core *c, const void *in, void *out) {
     if (st == MOFFT_SUCCESS &&
         ((down != run && (cudaEventRecord(done, run) != cudaSuccess ||
                           cudaStreamWaitEvent(down, done, 0) != cudaSuccess)) ||
-         cudaMemcpyAsync((unsigned char *)out + off, dout, bytes, cudaMemcpyDeviceToHost,
-                         down) != cudaSuccess))
+         download(c, (unsigned char *)out + off, dout, b1 - b0, down) != cudaSuccess))
       st = MOFFT_INTERNAL_ERROR;
   }
   cudaStream_t streams[3] = {up, run, down};

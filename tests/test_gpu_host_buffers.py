@@ -34,3 +34,28 @@ def test_repeated_host_executes(n, batch, gap, bits):
                 lines = buf.reshape(batch, dist)[:, :n].astype(np.complex128)
                 got = out.reshape(batch, dist)[:, :n]
                 assert rel_l2(got, oracle.fft_ld(lines, m.BACKWARD)) <= tol, (placement, call)
+
+
+@pytest.mark.parametrize("n,batch,gap", [(16, 3, 1), (1000, 3, 5), (256, 200, 7), (32768, 2, 3),
+                                         (4096, 1000, 4)])
+@pytest.mark.parametrize("bits", [32, 64])
+def test_gaps_between_transforms_stay(n, batch, gap, bits):
+    """A strided host execute writes its transforms and nothing between them,
+    staged in one chunk or several (the last case) and on the mapped span."""
+    dist = n + gap
+    calls = (1, 2, 31, 32, 40) if batch * dist * bits // 4 <= 256 << 10 else (1, 2)
+    for placement in (m.OUT_OF_PLACE, m.IN_PLACE):
+        with m.Plan.create(n, m.FORWARD, placement, bits=bits, batch=batch,
+                           distance=dist) as plan:
+            for call in range(1, calls[-1] + 1):
+                buf = oracle.uniform(batch * dist, seed=call, dtype=CTYPE[bits])
+                out = buf.copy() if placement == m.IN_PLACE else np.full_like(buf, 3 - 5j)
+                plan.execute(out if placement == m.IN_PLACE else buf, out)
+                before = buf if placement == m.IN_PLACE else np.full_like(buf, 3 - 5j)
+                got = out.reshape(batch, dist)
+                assert np.array_equal(got[:, n:], before.reshape(batch, dist)[:, n:]), \
+                    (placement, call)
+                if call in calls:
+                    ref = oracle.fft_ld(buf.reshape(batch, dist)[:, :n].astype(np.complex128), -1)
+                    tol = fp32_tol(n) if bits == 32 else fp64_tol(n)
+                    assert rel_l2(got[:, :n], ref) <= tol, (placement, call)
