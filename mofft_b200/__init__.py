@@ -552,7 +552,11 @@ class Server:
 
 def fft(x, direction: int = FORWARD, *, inplace: bool = False):
     """Batched transform of a torch tensor of shape (..., n), complex64 or
-    complex128, on its CUDA device.  Returns the output tensor."""
+    complex128, on its CUDA device.  Returns the output tensor.
+
+    Runs in the order of torch's current stream.  On the default stream the
+    call returns after the transform has completed; on any other stream it
+    enqueues and returns."""
     import torch
     if not x.is_cuda:
         raise ValueError("fft() takes a CUDA tensor; use Plan for host arrays")
@@ -565,12 +569,23 @@ def fft(x, direction: int = FORWARD, *, inplace: bool = False):
     out = x if inplace else torch.empty_like(x)
     device = x.get_device()
     plan = _plan_cache_get(n, batch, direction, inplace, bits, device)
-    stream = torch.cuda.current_stream(device).cuda_stream or None
+    current = torch.cuda.current_stream(device)
+    stream = current.cuda_stream or _LEGACY_STREAM
     if plan._stream != stream:
         plan.set_stream(stream)
     plan.execute(x, out)
+    if stream == _LEGACY_STREAM:
+        if bits == 32:
+            plan.check_status()
+        else:  # no FP64 kernel keeps a status
+            current.synchronize()
     return out
 
+
+# cudaStreamLegacy: the default stream as an explicit handle.  Handle 0 would
+# leave a plan on its own non-blocking stream, which nothing orders behind the
+# default stream's pending work.
+_LEGACY_STREAM = 1
 
 _PLAN_CACHE: dict = {}
 
