@@ -2,6 +2,8 @@
 // mofft_cuda.h.  Each registry entry is one compiled variant (precision, line
 // length, threads per line, lines per CTA, in-CTA radix chain).  The host
 // planner picks entries; the MEASURE planner times them.
+#include <map>
+#include <tuple>
 #include <vector>
 
 #include "fft_instances.cuh"
@@ -39,6 +41,22 @@ extern "C" const mofft_kernel_desc *mofft_cuda_kernel_get(int index) {
   const auto &r = registry();
   if (index < 0 || index >= (int)r.size()) return nullptr;
   return &r[index].desc;
+}
+
+extern "C" int mofft_cuda_kernels_of(int kind, int precision_bits, int length,
+                                     const int **indices) {
+  using Key = std::tuple<int, int, int>;
+  static const std::map<Key, std::vector<int>> index = [] {
+    std::map<Key, std::vector<int>> m;
+    const auto &r = registry();
+    for (int i = 0; i < (int)r.size(); ++i)
+      m[Key(r[i].desc.kind, r[i].desc.precision_bits, r[i].desc.length)].push_back(i);
+    return m;
+  }();
+  const auto it = index.find(Key(kind, precision_bits, length));
+  if (it == index.end()) return 0;
+  *indices = it->second.data();
+  return (int)it->second.size();
 }
 
 extern "C" size_t mofft_cuda_generic_smem(int precision_bits, int length,

@@ -25,6 +25,7 @@
 #include <cuda_runtime_api.h>
 #include <errno.h>
 #include <float.h>
+#include <limits.h>
 #include <math.h>
 #include <stdatomic.h>
 #include <stdio.h>
@@ -218,15 +219,14 @@ static int generic_kernel_index(int precision_bits, unsigned bank, const int *ch
   for (int i = 0; i < count; ++i)
     if (chain[i] > max_radix) max_radix = chain[i];
   int best = -1, best_cap = 1 << 30;
-  const int n = mofft_cuda_kernel_count();
+  const int *of = NULL;
+  const int n = mofft_cuda_kernels_of(MOFFT_KERNEL_GENERIC, precision_bits, 0, &of);
   for (int i = 0; i < n; ++i) {
-    const mofft_kernel_desc *d = mofft_cuda_kernel_get(i);
-    if (d->kind != MOFFT_KERNEL_GENERIC || d->precision_bits != precision_bits ||
-        d->bank != (int)bank)
-      continue;
+    const mofft_kernel_desc *d = mofft_cuda_kernel_get(of[i]);
+    if (d->bank != (int)bank) continue;
     const int cap = d->radices[0];
     if (cap >= max_radix && cap < best_cap) {
-      best = i;
+      best = of[i];
       best_cap = cap;
     }
   }
@@ -247,19 +247,19 @@ static int find_special(int precision_bits, int kind, const int *chain,
                         int count, long long total, long long ns_outer) {
   long long length = 1;
   for (int i = 0; i < count; ++i) length *= chain[i];
-  const int n = mofft_cuda_kernel_count();
+  if (length > INT_MAX) return -1;
+  const int *of = NULL;
+  const int n = mofft_cuda_kernels_of(kind, precision_bits, (int)length, &of);
   for (int i = 0; i < n; ++i) {
-    const mofft_kernel_desc *d = mofft_cuda_kernel_get(i);
-    if (d->kind != kind || d->precision_bits != precision_bits ||
-        d->length != length || d->cluster > 0 ||
-        !chain_equal(d->radices, d->radix_count, chain, count))
+    const mofft_kernel_desc *d = mofft_cuda_kernel_get(of[i]);
+    if (d->cluster > 0 || !chain_equal(d->radices, d->radix_count, chain, count))
       continue;
     if (kind == MOFFT_KERNEL_COLS) {
       const long long lines_total = total / length;
       if (lines_total % d->lines != 0) continue;
       if (ns_outer != 1 && ns_outer % d->lines != 0) continue;
     }
-    return i;
+    return of[i];
   }
   return -1;
 }
@@ -491,6 +491,14 @@ int mofft_auto_radices(long long length, int *out, int capacity) {
   return n == 1 ? count : -1;
 }
 
+/* Instructions per point of the radix-R codelet (the generated list holds 2..16,
+ * 32 and 64 in this order). */
+static double codelet_cost(int radix) {
+  _Static_assert(MOFFT_CODELET_COST_COUNT == 17, "radices 2..16, 32, 64");
+  const int i = radix <= 16 ? radix - 2 : radix == 32 ? 15 : 16;
+  return (double)k_mofft_codelet_costs[i].instr / radix;
+}
+
 /* Cost of a runtime-chain line DFT, in instructions per point: each stage's
  * codelet, 12 for the exchange, barrier and twiddles of a stage boundary, and a
  * penalty as the points resident per SM fall below 96 KB.  Fitted to timings of
@@ -505,10 +513,7 @@ static double runtime_chain_cost(int precision_bits, int cols, long long length,
                                &lines, &threads, &smem, &ctas))
     return 1e6 + count;
   double cost = 12.0 * (count - 1);
-  for (int i = 0; i < count; ++i)
-    for (int k = 0; k < MOFFT_CODELET_COST_COUNT; ++k)
-      if (k_mofft_codelet_costs[k].radix == chain[i])
-        cost += (double)k_mofft_codelet_costs[k].instr / chain[i];
+  for (int i = 0; i < count; ++i) cost += codelet_cost(chain[i]);
   const double resident = (double)ctas * lines * (double)length *
                           (double)mofft_complex_bytes(precision_bits) / 98304.0;
   if (resident < 1.0) cost += 16.0 * (1.0 / resident - 1.0);
@@ -533,7 +538,12 @@ typedef struct {
   double best_cost;
 } chain_search;
 
-static void search_runtime_chain(chain_search *s, long long rest, int most, int count) {
+/* The chains below chain[0..count), whose stages cost `spent`.  A chain of rest
+ * more points costs at least 2 per factor of two (no codelet takes less: 2, 4 and
+ * 8 points take 2, 4 and 7) and 12 per stage boundary, which ends most
+ * branches before the tile rule prices a leaf. */
+static void search_runtime_chain(chain_search *s, long long rest, int most, int count,
+                                 double spent) {
   if (rest == 1) {
     const double cost = runtime_chain_cost(s->precision_bits, s->cols, s->length,
                                            s->line_units, s->chain, count);
@@ -545,10 +555,13 @@ static void search_runtime_chain(chain_search *s, long long rest, int most, int 
     return;
   }
   if (count >= 8) return;
+  const int bits = 63 - __builtin_clzll((unsigned long long)rest);   /* whole factors of 2 */
+  const double least = spent + 12.0 * (count + (bits + 3) / 4 - 1) + 2.0 * bits;
+  if (least - 1e-9 > s->best_cost) return;
   for (int r = most; r >= 2; --r) {
     if (rest % r) continue;
     s->chain[count] = r;
-    search_runtime_chain(s, rest / r, r, count + 1);
+    search_runtime_chain(s, rest / r, r, count + 1, spent + codelet_cost(r));
   }
 }
 
@@ -563,10 +576,35 @@ static int runtime_chain(int precision_bits, int cols, long long length, long lo
   s.length = length;
   s.line_units = line_units;
   s.best_cost = 1e6;
-  search_runtime_chain(&s, length, 16, 0);
+  search_runtime_chain(&s, length, 16, 0, 0.0);
   if (s.best_count <= 0 || s.best_count > capacity) return 0;
   memcpy(out, s.best, (size_t)s.best_count * sizeof(int));
   return s.best_count;
+}
+
+/* The runtime column chains of one transform's splits by line length: the same
+ * few hundred lengths recur in every split. */
+#define CHAIN_MEMO 1024
+typedef struct {
+  int length, count;      /* count: runtime_chain's, 0 = none fits */
+  int chain[8];
+} chain_memo;
+
+static int remembered_chain(chain_memo *memo, int precision_bits, long long length,
+                            long long line_units, int *out, int capacity) {
+  unsigned at = (unsigned)length * 2654435761u >> 22;
+  for (int probe = 0; memo && probe < CHAIN_MEMO; ++probe, at = (at + 1) % CHAIN_MEMO) {
+    chain_memo *m = memo + at;
+    if (m->length == 0) {
+      m->length = (int)length;
+      m->count = runtime_chain(precision_bits, 1, length, line_units, m->chain, 8);
+    }
+    if (m->length != length) continue;
+    if (m->count > capacity) return 0;
+    memcpy(out, m->chain, (size_t)m->count * sizeof(int));
+    return m->count;
+  }
+  return runtime_chain(precision_bits, 1, length, line_units, out, capacity);
 }
 
 /* Preferred chain of a pass of length L: the first registered specialised
@@ -574,14 +612,15 @@ static int runtime_chain(int precision_bits, int cols, long long length, long lo
  * else the generic default chain. */
 static int preferred_chain(int precision_bits, unsigned bank, int kind,
                            long long length, long long total,
-                           long long ns_outer, int *out, int capacity) {
+                           long long ns_outer, chain_memo *memo, int *out, int capacity) {
   if (bank == 0) {
-    const int n = mofft_cuda_kernel_count();
+    const int *of = NULL;
+    const int n = length <= INT_MAX
+                      ? mofft_cuda_kernels_of(kind, precision_bits, (int)length, &of)
+                      : 0;
     for (int i = 0; i < n; ++i) {
-      const mofft_kernel_desc *d = mofft_cuda_kernel_get(i);
-      if (d->kind != kind || d->precision_bits != precision_bits ||
-          d->length != length || d->radix_count > capacity || d->cluster > 0)
-        continue;
+      const mofft_kernel_desc *d = mofft_cuda_kernel_get(of[i]);
+      if (d->radix_count > capacity || d->cluster > 0) continue;
       if (kind == MOFFT_KERNEL_COLS) {
         if ((total / length) % d->lines != 0) continue;
         if (ns_outer != 1 && ns_outer % d->lines != 0) continue;
@@ -590,9 +629,10 @@ static int preferred_chain(int precision_bits, unsigned bank, int kind,
       return d->radix_count;
     }
     if (length <= 16384) {
-      const int cols = kind == MOFFT_KERNEL_COLS;
-      const int count = runtime_chain(precision_bits, cols, length, cols ? total / length : 1,
-                                      out, capacity);
+      const int count =
+          kind == MOFFT_KERNEL_COLS
+              ? remembered_chain(memo, precision_bits, length, total / length, out, capacity)
+              : runtime_chain(precision_bits, 0, length, 1, out, capacity);
       if (count > 0) return count;
     }
   }
@@ -664,10 +704,7 @@ static double split_cost(int precision_bits, unsigned bank, size_t length, size_
       return 1e6;
     }
     double cost = 60.0 + 8.0 * (ps->radix_count - 1);
-    for (int i = 0; i < ps->radix_count; ++i)
-      for (int k = 0; k < MOFFT_CODELET_COST_COUNT; ++k)
-        if (k_mofft_codelet_costs[k].radix == ps->radices[i])
-          cost += (double)k_mofft_codelet_costs[k].instr / ps->radices[i];
+    for (int i = 0; i < ps->radix_count; ++i) cost += codelet_cost(ps->radices[i]);
     const double resident = (double)ctas * lines * (double)ps->length * cb / 65536.0;
     if (resident < 1.0) cost += 8.0 * (1.0 / resident - 1.0);
     total += runtime ? 1.4 * cost : cost;
@@ -697,8 +734,8 @@ static int model_chain(int precision_bits, unsigned bank, size_t length, int *ch
   mofft_schedule sched;
   /* one pass */
   int count = one_pass ? preferred_chain(precision_bits, bank, MOFFT_KERNEL_ROWS,
-                                         (long long)length, (long long)length, 1, chain,
-                                         capacity)
+                                         (long long)length, (long long)length, 1, NULL,
+                                         chain, capacity)
                        : 0;
   if (count > 0 && mofft_group_chain(precision_bits, bank, chain, count,
                                      (long long)length, &sched) &&
@@ -717,6 +754,7 @@ static int model_chain(int precision_bits, unsigned bank, size_t length, int *ch
   const long long n = (long long)length;
   collect_divisors(n, 2, 1 << 16, divs, &ndiv, kMaxDiv);
   const size_t model_batch = n >= (1LL << 25) ? 1 : (size_t)((1LL << 25) / n);
+  chain_memo *memo = calloc(CHAIN_MEMO, sizeof(*memo)); /* without it each is searched anew */
   ranked_split kept[kKeep];
   int nkept = 0;
   for (int passes = 2; passes <= 3 && nkept == 0; ++passes) {
@@ -739,7 +777,7 @@ static int model_chain(int precision_bits, unsigned bank, size_t length, int *ch
         for (int p = 0; p < passes && ok; ++p) {
           if (L[p] < 2 || L[p] > (1 << 16)) { ok = 0; break; }
           const int k = preferred_chain(precision_bits, bank, MOFFT_KERNEL_COLS, L[p], n, ns,
-                                        c.chain + c.count, MOFFT_MAX_STAGES - c.count);
+                                        memo, c.chain + c.count, MOFFT_MAX_STAGES - c.count);
           if (k <= 0) { ok = 0; break; }
           c.count += k;
           if (p < passes - 1) cuts[p] = c.count;
@@ -759,6 +797,7 @@ static int model_chain(int precision_bits, unsigned bank, size_t length, int *ch
       }
     }
   }
+  free(memo);
   int best = -1;
   for (int i = 0; i < nkept; ++i) {
     if (!mofft_group_chain(precision_bits, bank, kept[i].chain, kept[i].count, n, &sched))

@@ -84,6 +84,11 @@ typedef struct {
 
 int mofft_cuda_kernel_count(void);
 const mofft_kernel_desc *mofft_cuda_kernel_get(int index);
+/* Registry indices of a kind, precision and line length (0 for the generic
+ * kernels) in registry order; returns their number.  The planner asks this for
+ * every pass of every split. */
+int mofft_cuda_kernels_of(int kind, int precision_bits, int length,
+                          const int **indices);
 /* Dynamic shared memory the generic kernel needs for (L, lines, cols). */
 size_t mofft_cuda_generic_smem(int precision_bits, int length, int lines,
                                int cols);

@@ -465,3 +465,18 @@ def test_every_smooth_length_has_a_schedule():
             assert s["pass_count"] <= 3
             assert all(0 < b <= 227 * 1024 for b in s["smem_bytes"])
             assert all(2 <= r <= 16 or r in (32, 64) for r in s["radices"])
+
+
+@pytest.mark.parametrize("n,bits", [(362880, 32), (604800, 64), (720720, 32)])
+def test_planning_stays_short(n, bits):
+    """Lengths without wisdom: choosing splits and chains is part of every plan
+    creation.  About 1.2 ms each where this was written; every split searching
+    its chains anew took 5.7 to 7.3 ms there, and cost as much as several
+    transforms."""
+    import time
+    best = 1e9
+    for _ in range(20):
+        t = time.perf_counter()
+        m.schedule_preview(n, bits)
+        best = min(best, time.perf_counter() - t)
+    assert best < 3.5e-3
