@@ -336,7 +336,6 @@ class Plan:
         self._s = "f32" if bits == 32 else "f64"
         self._lib = load()
         self._execute = self._fn("execute")
-        self._stream: Optional[int] = None
 
     def _fn(self, name: str):
         return getattr(self._lib, f"mofft_{name}_{self._s}")
@@ -386,7 +385,6 @@ class Plan:
 
     def set_stream(self, stream_handle: Optional[int]) -> None:
         check(self._fn("plan_set_stream")(self._h, stream_handle or None), "set_stream")
-        self._stream = stream_handle or None
 
     def set_kernel_bank(self, bank: int) -> None:
         check(self._fn("plan_set_kernel_bank")(self._h, bank), "set_kernel_bank")
@@ -568,11 +566,9 @@ def fft(x, direction: int = FORWARD, *, inplace: bool = False):
     bits = 32 if x.dtype == torch.complex64 else 64
     out = x if inplace else torch.empty_like(x)
     device = x.get_device()
-    plan = _plan_cache_get(n, batch, direction, inplace, bits, device)
     current = torch.cuda.current_stream(device)
     stream = current.cuda_stream or _LEGACY_STREAM
-    if plan._stream != stream:
-        plan.set_stream(stream)
+    plan = _plan_cache_get(n, batch, direction, inplace, bits, device, stream)
     plan.execute(x, out)
     if stream == _LEGACY_STREAM:
         if bits == 32:
@@ -590,11 +586,16 @@ _LEGACY_STREAM = 1
 _PLAN_CACHE: dict = {}
 
 
-def _plan_cache_get(n, batch, direction, inplace, bits, device):
-    key = (n, batch, direction, inplace, bits, device)
+def _plan_cache_get(n, batch, direction, inplace, bits, device, stream):
+    """The plan of a shape on a stream.  A plan stays on the stream it was made
+    for: plans of several passes may own a workspace, which calls on one
+    stream use in turn and calls on two streams would overwrite for each
+    other."""
+    key = (n, batch, direction, inplace, bits, device, stream)
     plan = _PLAN_CACHE.get(key)
     if plan is None:
         plan = Plan.create(n, direction, IN_PLACE if inplace else OUT_OF_PLACE,
                            bits=bits, batch=batch)
-        _PLAN_CACHE[key] = plan
+        plan.set_stream(stream)
+        plan = _PLAN_CACHE.setdefault(key, plan)  # another thread's may be first
     return plan

@@ -1487,7 +1487,11 @@ mofft_status mofft_core_execute(const mofft_core *cc, const void *in, void *out)
   const int dev_out = in == out ? dev_in : is_device_pointer(out);
   void *stream = c->user_stream ? c->user_stream : c->stream;
   if (dev_in && dev_out) {
+    /* another thread's passes must not come between two that share the
+     * workspace */
+    if (c->d_work) pthread_mutex_lock(&c->lock);
     st = mofft_core_enqueue(c, in, out, stream);
+    if (c->d_work) pthread_mutex_unlock(&c->lock);
     if (st == MOFFT_SUCCESS && !c->user_stream &&
         cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) {
       cudaGetLastError();

@@ -79,6 +79,56 @@ def test_default_stream_keeps_its_order(fakes, bits):
     assert plan.log[1:] == ([("wait", 1)] if bits == 32 else []) and waits == [0] * (bits == 64)
 
 
+def test_streams_do_not_share_a_plan(fakes):
+    """A plan may own a workspace: no plan runs on two streams, and a stream's
+    second call finds its plan again."""
+    import torch
+    x = FakeTensor(65536, torch.complex64)
+    for handle in (7, 9, 0, 7, 9, 0):
+        fakes(handle)
+        m.fft(x, inplace=True)
+    ran = [[s for what, s in p.log if what == "run"] for p in FakePlan.made]
+    assert ran == [[7, 7], [9, 9], [1, 1]]
+
+
+def test_threads_do_not_move_each_others_stream(fakes, monkeypatch):
+    """Two threads on two streams, the second calling while the first one is
+    inside its call: each transform runs on its own thread's stream."""
+    import threading
+    import torch
+    local = threading.local()
+    monkeypatch.setattr(torch.cuda, "current_stream",
+                        lambda device=None: types.SimpleNamespace(cuda_stream=local.handle))
+    seen, lock = [], threading.Lock()
+    real = FakePlan.execute
+
+    def execute(self, inp, out=None):
+        real(self, inp, out)
+        with lock:
+            seen.append((local.handle, self._stream))
+    monkeypatch.setattr(FakePlan, "execute", execute)
+    real_set, turn = FakePlan.set_stream, threading.Barrier(2, timeout=2)
+
+    def set_stream(self, stream):
+        real_set(self, stream)
+        try:                                  # both threads have set theirs
+            turn.wait()
+        except threading.BrokenBarrierError:
+            pass
+    monkeypatch.setattr(FakePlan, "set_stream", set_stream)
+
+    def work(handle):
+        local.handle = handle
+        for _ in range(50):
+            m.fft(FakeTensor(65536, torch.complex64), inplace=True)
+    threads = [threading.Thread(target=work, args=(h,)) for h in (7, 9)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(seen) == 100 and all(a == b for a, b in seen)
+
+
 @pytest.mark.gpu
 @needs_gpu
 @pytest.mark.parametrize("n,batch,bits", [(1024, 1, 32), (16384, 3, 32), (65536, 4, 32),
@@ -98,3 +148,48 @@ def test_default_stream_waits_for_the_input(n, batch, bits, inplace):
     y = m.fft(x, inplace=inplace)
     ref = oracle.fft_ld(host.astype(np.complex128), -1)
     assert rel_l2(y.cpu().numpy(), ref) <= (fp32_tol(n) if bits == 32 else fp64_tol(n))
+
+
+@pytest.mark.gpu
+@needs_gpu
+@pytest.mark.parametrize("n,batch,bits,inplace", [(65536, 64, 32, True), (50625, 40, 64, True),
+                                                  (1 << 24, 1, 32, False),
+                                                  (1 << 23, 1, 64, False)])
+def test_streams_with_a_workspace(n, batch, bits, inplace):
+    """Transforms of several passes with a workspace, on three streams at once
+    (one of them the default one) and from two threads on one stream."""
+    import threading
+    import torch
+    dtype = torch.complex64 if bits == 32 else torch.complex128
+    real = torch.float32 if bits == 32 else torch.float64
+    g = torch.Generator(device="cuda").manual_seed(n)
+
+    def data():
+        return torch.view_as_complex(torch.rand((batch, n, 2), generator=g, device="cuda",
+                                                dtype=real) * 2 - 1)
+    xs = [data() for _ in range(3)]
+    refs = [m.fft(x) for x in xs]             # one at a time
+    streams = [torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.default_stream()]
+
+    def run(x, stream, out):
+        with torch.cuda.stream(stream):
+            out.extend(m.fft(x.clone() if inplace else x, inplace=inplace) for _ in range(4))
+    outs = [[], [], []]
+    for x, s in zip(xs, streams):
+        s.wait_stream(torch.cuda.default_stream())
+        run(x, s, outs[0])                    # make the plans
+    torch.cuda.synchronize()
+    for where in (streams, [streams[0]] * 2 + [streams[1]]):
+        outs = [[], [], []]
+        threads = [threading.Thread(target=run, args=a) for a in zip(xs, where, outs)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        for ref, got in zip(refs, outs):
+            assert len(got) == 4
+            for y in got:
+                err = torch.linalg.vector_norm(y - ref) / torch.linalg.vector_norm(ref)
+                # the same kernels on the same input; in place may run another schedule
+                assert float(err) <= (fp32_tol(n) if bits == 32 else fp64_tol(n))
