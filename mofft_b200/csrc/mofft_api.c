@@ -1356,9 +1356,11 @@ static mofft_status ensure_staging(mofft_core *c, size_t chunks) {
  * KiB in 51 instead of 73.  Beyond that the host's own copies take most of a
  * call and the gain shrinks to the spread between hosts (400 to 500 KiB: 91 to
  * 114 us on both paths, one host 25 % slower on this one).
- * Allocating that memory takes 1.3 to 3 ms, some hundred times the saving: a
- * plan does it at its 32nd such call, so plans that run a few times never pay
- * it. */
+ * The memory holds the plan's own span twice, input then output, and goes with
+ * the plan.  The driver cuts it from chunks of 2 MiB: a new chunk takes it 1.2
+ * to 3 ms, some hundred times the saving of a call, room in one a few us.  A
+ * plan asks for it at its 32nd such call, so plans that run a few times never
+ * pay it, and 64 plans of 1024 FP32 points share one chunk. */
 #define MOFFT_PINNED_SPAN ((size_t)256 << 10)
 #define MOFFT_PINNED_CALLS 32u
 
@@ -1368,8 +1370,8 @@ static int runs_on_host_memory(mofft_core *c, size_t span) {
   if (span > MOFFT_PINNED_SPAN || c->sched.pass_count != 1 || schedule_has_status(c)) return 0;
   if (c->h_pinned) return 1;
   if (++c->small_host_calls < MOFFT_PINNED_CALLS) return 0;
-  /* one allocation, input then output; without it the calls stay staged */
-  if (cudaHostAlloc(&c->h_pinned, 2 * MOFFT_PINNED_SPAN, cudaHostAllocMapped) != cudaSuccess) {
+  /* without it the calls stay staged */
+  if (cudaHostAlloc(&c->h_pinned, 2 * align256(span), cudaHostAllocMapped) != cudaSuccess) {
     cudaGetLastError();
     c->h_pinned = NULL;
     c->small_host_calls = 0;
@@ -1379,7 +1381,7 @@ static int runs_on_host_memory(mofft_core *c, size_t span) {
 }
 
 static mofft_status execute_pinned(mofft_core *c, const void *in, void *out, size_t span) {
-  unsigned char *src = (unsigned char *)c->h_pinned, *dst = src + MOFFT_PINNED_SPAN;
+  unsigned char *src = (unsigned char *)c->h_pinned, *dst = src + align256(span);
   const size_t cb = mofft_complex_bytes(c->precision_bits);
   const size_t line = c->length * cb, pitch = c->distance * cb;
   memcpy(src, in, span);

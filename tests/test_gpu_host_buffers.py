@@ -59,3 +59,23 @@ def test_gaps_between_transforms_stay(n, batch, gap, bits):
                     ref = oracle.fft_ld(buf.reshape(batch, dist)[:, :n].astype(np.complex128), -1)
                     tol = fp32_tol(n) if bits == 32 else fp64_tol(n)
                     assert rel_l2(got[:, :n], ref) <= tol, (placement, call)
+
+
+def test_mapped_memory_fits_the_plan():
+    """64 small plans past their 32nd host call: 16 KiB of mapped memory each,
+    which the driver cuts from chunks of 2 MiB."""
+    def shared_kib():
+        with open("/proc/self/status") as f:
+            return next(int(line.split()[1]) for line in f if line.startswith("RssShmem"))
+
+    x = oracle.uniform(1024, seed=1, dtype=np.complex64)
+    out = np.empty_like(x)
+    plans = [m.Plan.create(1024) for _ in range(64)]
+    for plan in plans:
+        for _ in range(31):
+            plan.execute(x, out)
+    before = shared_kib()
+    for plan in plans:
+        plan.execute(x, out)
+    assert shared_kib() - before <= 2 * 2048
+    assert rel_l2(out, oracle.fft_ld(x.astype(np.complex128), -1)) <= fp32_tol(1024)
