@@ -23,19 +23,10 @@ bool rt_pass_shape(const mofft_pass_args *p, RtShape *s) {
 // several-butterfly kernels.
 template <typename T, int MODE>
 const void *rt_func(int max_radix, bool multi) {
-  constexpr int bits = sizeof(T) == 4 ? 32 : 64;
-  constexpr bool cols = MODE >= kRtColsHead;
-  if (multi)
-    return reinterpret_cast<const void *>(
-        &rt_kernel<T, MODE, 16, true, rt_max_threads(bits, cols, 16, true)>);
-  if (max_radix <= 8)
-    return reinterpret_cast<const void *>(
-        &rt_kernel<T, MODE, 8, false, rt_max_threads(bits, cols, 8, false)>);
-  if (max_radix <= 11)
-    return reinterpret_cast<const void *>(
-        &rt_kernel<T, MODE, 11, false, rt_max_threads(bits, cols, 11, false)>);
-  return reinterpret_cast<const void *>(
-      &rt_kernel<T, MODE, 16, false, rt_max_threads(bits, cols, 16, false)>);
+  if (multi) return reinterpret_cast<const void *>(&rt_kernel<T, MODE, 16, true>);
+  if (max_radix <= 8) return reinterpret_cast<const void *>(&rt_kernel<T, MODE, 8, false>);
+  if (max_radix <= 11) return reinterpret_cast<const void *>(&rt_kernel<T, MODE, 11, false>);
+  return reinterpret_cast<const void *>(&rt_kernel<T, MODE, 16, false>);
 }
 
 template <typename T>

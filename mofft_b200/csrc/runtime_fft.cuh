@@ -29,14 +29,17 @@
 // at n = 343 before the stages were peeled), HBM for the short lengths that
 // run direct.  Measured per 2^25 FP32 / 2^24 FP64 points (HBM floor 82 us),
 // this against the ping-pong kernel: FP32 n = 100 801 -> 98 us, 343 1397 ->
-// 117, 1000 1005 -> 122, 3375 976 -> 128, 10000 1441 -> 214, 50625 (two
-// passes) 1849 -> 262; FP64 100 476 -> 86, 3375 672 -> 135, 50625 1233 -> 224.
-// Rel-L2 errors against 64 bits are those of the chain's codelets plus one
-// product per twiddle: FP32 3375 1.30e-7 -> 1.36e-7, 248832 1.92e-7 ->
-// 1.84e-7; FP64 3375 4.1e-16 -> 4.2e-16.
+// 117, 1000 1005 -> 122, 3375 976 -> 133, 10000 1441 -> 218, 50625 (two
+// passes) 1849 -> 292; FP64 100 476 -> 86, 3375 672 -> 136, 50625 1233 -> 237.
+// Every stage twiddle is looked up.  Deriving most of them as products of two
+// others (6 loads instead of 15 at radix 16) took 0.4 % less time over 72
+// lengths, 2 to 4 % less at these, but added 2 to 5 % to the rel-L2 error: FP32
+// 343 1.062e-7 -> 1.092e-7, 3375 1.314e-7 -> 1.360e-7, FP64 343 1.937e-16 ->
+// 1.977e-16.
 #pragma once
 
 #include "fft_device.cuh"
+#include "runtime_tile.h"
 
 namespace mofft {
 
@@ -83,27 +86,14 @@ __device__ __forceinline__ int rt_div(int n, unsigned m) {
   return m ? (int)__umulhi((unsigned)n, m) : n;
 }
 
-// Stage twiddles v[r] *= w^r.  w^1 .. w^4, w^8 and w^12 come from the table,
-// every other power is one product of two of them (w^4q * w^k), so a radix-16
-// butterfly needs 6 loads instead of 15 and no power carries more than one
-// extra rounding (every power from the table: 2-6 % slower, the error 1-4 %
-// smaller).
+// Stage twiddles v[r] *= w^r, every power from the table.
 template <typename T, int R>
 __device__ __forceinline__ void rt_twiddle(T (&vr)[R], T (&vi)[R],
                                            const cplx_t<T>* __restrict__ tw, int ns) {
-  T wr[R], wi[R];
 #pragma unroll
   for (int r = 1; r < R; ++r) {
-    if (r <= 3 || r % 4 == 0) {
-      const cplx_t<T> w = __ldg(tw + (r - 1) * ns);
-      wr[r] = w.x;
-      wi[r] = w.y;
-    } else {
-      const int h = r / 4 * 4, l = r % 4;
-      wr[r] = wr[h] * wr[l] - wi[h] * wi[l];
-      wi[r] = wr[h] * wi[l] + wi[h] * wr[l];
-    }
-    cmul<T>(vr[r], vi[r], wr[r], wi[r]);
+    const cplx_t<T> w = __ldg(tw + (r - 1) * ns);
+    cmul<T>(vr[r], vi[r], w.x, w.y);
   }
 }
 
@@ -315,8 +305,14 @@ __device__ __forceinline__ void rt_dispatch(const RtTile<T, MODE>& tile, const R
 #undef MOFFT_RT_CASE
 }
 
-template <typename T, int MODE, int MAXR, bool MULTI, int MAXT>
-__global__ void __launch_bounds__(MAXT, 1) rt_kernel(const __grid_constant__ RtArgs<T> a) {
+// Registers are capped at the figures the planner's occupancy rests on
+// (rt_registers), which every form meets without spills; uncapped, looking up all
+// twiddles takes 56 to 64 where 48 and 56 do (FP32 1764 139 against 126 us of
+// 2^25 points).
+template <typename T, int MODE, int MAXR, bool MULTI>
+__global__ void __maxnreg__((rt_registers(sizeof(T) == 4 ? 32 : 64, MODE >= kRtColsHead, MAXR,
+                                          MULTI)))
+rt_kernel(const __grid_constant__ RtArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx_t<T>* sp = reinterpret_cast<cplx_t<T>*>(smem_raw);
   constexpr bool COLS = MODE >= kRtColsHead;

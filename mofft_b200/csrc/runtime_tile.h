@@ -7,21 +7,9 @@
 
 namespace mofft {
 
-// Most threads of a CTA: the launch bounds of the register class that runs a
-// chain's largest radix.  The register file divided by them is at or above
-// what the class needs unspilled (-Xptxas -v: FP32 37 / 48 / 63 registers for
-// radices up to 8 / 11 / 16, up to 80 in column passes with super-stage
-// twiddles; FP64 64 / 80 / 106, column passes 84 / 110 / 124).
-constexpr int rt_max_threads(int precision_bits, bool cols, int max_radix, bool multi) {
-  if (multi) return precision_bits == 32 ? (cols ? 768 : 1024) : 512;
-  if (precision_bits == 32) return max_radix <= 11 || !cols ? 1024 : 768;
-  if (max_radix <= 8) return cols ? 640 : 1024;
-  if (max_radix <= 11) return cols ? 512 : 768;
-  return 512;
-}
-
-// Registers per thread of those kernels as compiled (the larger of the first
-// and later column passes), for the planner's occupancy.
+// Registers per thread of the kernels by register class (the chain's largest
+// radix up to 8, 11, 16, or several butterflies): their cap when compiled, and
+// the planner's occupancy.
 constexpr int rt_registers(int precision_bits, bool cols, int max_radix, bool multi) {
   if (precision_bits == 32) {
     if (multi) return cols ? 80 : 64;
@@ -30,6 +18,29 @@ constexpr int rt_registers(int precision_bits, bool cols, int max_radix, bool mu
   if (multi) return cols ? 128 : 112;
   return max_radix <= 8 ? (cols ? 72 : 64) : max_radix <= 11 ? (cols ? 88 : 80) : cols ? 128 : 104;
 }
+
+// Most threads of a CTA: what the register file holds of the class, in steps
+// of the tile rule's timings.
+constexpr int rt_max_threads(int precision_bits, bool cols, int max_radix, bool multi) {
+  if (multi) return precision_bits == 32 ? (cols ? 768 : 1024) : 512;
+  if (precision_bits == 32) return max_radix <= 11 || !cols ? 1024 : 768;
+  if (max_radix <= 8) return cols ? 640 : 1024;
+  if (max_radix <= 11) return cols ? 512 : 768;
+  return 512;
+}
+
+// A CTA of the most threads fits the register file in every class.
+constexpr bool rt_threads_fit() {
+  for (int bits = 32; bits <= 64; bits += 32)
+    for (int cols = 0; cols < 2; ++cols)
+      for (int radix : {8, 11, 16})
+        for (int multi = 0; multi < 2; ++multi)
+          if (rt_registers(bits, cols != 0, radix, multi != 0) *
+                  rt_max_threads(bits, cols != 0, radix, multi != 0) > 65536)
+            return false;
+  return true;
+}
+static_assert(rt_threads_fit(), "launch would exceed the register file");
 
 struct RtShape {
   int lines;       // lines per CTA
