@@ -286,7 +286,8 @@ struct GenericInst {
 
 
 // ST: true/false (staged I/O); ROWSD: staged flag plus derived radix-16
-// twiddles (name suffix _d).
+// twiddles (name suffix _d); ROWSDP / ROWSTP: pair exchanges with derived
+// twiddles or with looked-up ones (_dp, _p).
 #define ROWS(T, L, TPL, TB, ST, ...) \
   RowsInst<T, L, TPL, TB, (ST) ? kStaged : 0, __VA_ARGS__>::entry( \
       "rows_" #T "_" #L "_t" #TPL "_b" #TB "_s" #ST)
@@ -296,6 +297,9 @@ struct GenericInst {
 #define ROWSDP(T, L, TPL, TB, ...) \
   RowsInst<T, L, TPL, TB, kDerivedTw | kPairX, __VA_ARGS__>::entry( \
       "rows_" #T "_" #L "_t" #TPL "_b" #TB "_sfalse_dp")
+#define ROWSTP(T, L, TPL, TB, ...) \
+  RowsInst<T, L, TPL, TB, kPairX, __VA_ARGS__>::entry( \
+      "rows_" #T "_" #L "_t" #TPL "_b" #TB "_sfalse_p")
 #define ROWSDP0(T, L, TPL, TB, ...) \
   RowsInst<T, L, TPL, TB, kDerivedTw | kPairX | kPairPad0, __VA_ARGS__>::entry( \
       "rows_" #T "_" #L "_t" #TPL "_b" #TB "_sfalse_dp0")

@@ -6,7 +6,7 @@
 // butterflies do not divide evenly) and as many registers.  Here the odd factor
 // sits inside a radix of 10 or 12 (or a radix of its own with two to four
 // butterflies a thread) behind a radix-16 or radix-8 stage: at most 16 points
-// and 32 to 48 registers a thread (64 to 70 before).  A power of two first also
+// and 32 to 48 registers a thread in FP32 (64 to 70 before), up to 108 in FP64.  A power of two first also
 // makes the pad every 16 pairs free of bank conflicts (a bank simulation:
 // 1.0-1.2 wavefronts per access against 1.35-1.9).  Lengths below 400 used to
 // copy their lines through shared memory on both sides; reading and writing
@@ -18,7 +18,10 @@
 // 64 96 -> 82, 128 93 -> 81, 192 107 -> 84, 320 132 -> 90, 384 120 -> 87, 640
 // 100 -> 89, 1280 119 -> 93, 2048 99 -> 88, 6144 168 -> 156.
 // Tuned FP32 plans of 64, 320, 384, 1280 and 1536 points have moved on to the
-// two-line kernels of twin_fft.cuh (77, 89, 78, 85 and 80 us).
+// two-line kernels of twin_fft.cuh (80, 90, 85, 88 and 83 us).  FP64 128 looks
+// its radix-16 twiddles up (ROWSTP), as the kernel that it replaced did: derived
+// from four of them its rel-L2 error was 5 % larger (1.62e-16 -> 1.70e-16) for
+// 80.6 instead of 81.7 us.
 #include "fft_instances.cuh"
 
 namespace mofft {
@@ -46,7 +49,7 @@ const Entry *entries_rows_even(int *count) {
       ROWSDP(double, 320, 64, 2, 8, 5, 8),
       ROWSDP(double, 192, 16, 8, 16, 12),
       ROWSDP(double, 160, 16, 8, 16, 10),
-      ROWSDP(double, 128, 16, 8, 8, 16),
+      ROWSTP(double, 128, 16, 8, 8, 16),
       ROWSDP(double, 96, 12, 16, 8, 12),
       ROWSDP(double, 80, 10, 16, 8, 10),
       ROWSDP(double, 64, 8, 16, 8, 8),

@@ -19,6 +19,13 @@
 // registers: a pair halves the resident CTAs, whose barriers then show (4096
 // 170 -> 181, 8192 223 -> 291, 3072 171 -> 189, 2560 177 -> 205), nor where it
 // loses in L2 (160, 192, 640, 768, 1024, 2048).
+//
+// Every stage twiddle is looked up.  Forming powers above w^3 as products took
+// 1 % less time (5 % at 48 and 384: 95 -> 91, 85 -> 81 us of 2^25 points) and
+// made the rel-L2 errors of 64, 128 and 256 points 5 % larger than the one-line
+// kernels' (8.05e-8 -> 8.49e-8, 8.76e-8 -> 9.15e-8, 9.54e-8 -> 9.99e-8).  Looked
+// up they are 8.05e-8, 8.75e-8 and 9.52e-8, and 320-1536 points are 7 to 10 %
+// below the one-line kernels'.
 #pragma once
 
 #include "fft_device.cuh"
@@ -168,30 +175,15 @@ __device__ __forceinline__ void twin_rotate(Twin& xr, Twin& xi, float wr, float 
   xi = i;
 }
 
-// Stage twiddles v[r] *= w^r.  Radix 16: w^1 .. w^4, w^8, w^12 from the table,
-// the others one product (computed once for both lines).
+// Stage twiddles v[r] *= w^r, every power from the table: one load for both
+// lines.
 template <int R, int NS>
 __device__ __forceinline__ void twin_twiddle(Twin (&vr)[R], Twin (&vi)[R],
                                              const float2* __restrict__ tw) {
-  float2 low[4];
 #pragma unroll
-  for (int k = 1; k < 4; ++k)
-    if (k < R) low[k] = __ldg(tw + (k - 1) * NS);
-#pragma unroll
-  for (int q = 0; q < R; q += 4) {
-    float2 base;
-    if (q > 0) {
-      base = __ldg(tw + (q - 1) * NS);
-      twin_rotate(vr[q], vi[q], base.x, base.y);
-    }
-#pragma unroll
-    for (int k = 1; k < 4; ++k) {
-      if (q + k < R) {
-        float wr = low[k].x, wi = low[k].y;
-        if (q > 0) cmul<float>(wr, wi, base.x, base.y);
-        twin_rotate(vr[q + k], vi[q + k], wr, wi);
-      }
-    }
+  for (int r = 1; r < R; ++r) {
+    const float2 w = __ldg(tw + (r - 1) * NS);
+    twin_rotate(vr[r], vi[r], w.x, w.y);
   }
 }
 
