@@ -205,8 +205,10 @@ size_t generic_smem(int L, int lines, int cols) {
 // cudaErrorNotSupported when a pass's chain does not fit them.
 cudaError_t rt_launch_f32(const mofft_pass_args *p, cudaStream_t s);
 cudaError_t rt_launch_f64(const mofft_pass_args *p, cudaStream_t s);
-cudaError_t rt_prepare_f32();
-cudaError_t rt_prepare_f64();
+cudaError_t rt_prepare_f32(const mofft_pass_args *p);
+cudaError_t rt_prepare_f64(const mofft_pass_args *p);
+cudaError_t rt_prepare_columns_f32();
+cudaError_t rt_prepare_columns_f64();
 
 template <typename T, bool WIDE, int BANK = 0>
 struct GenericInst {

@@ -2,7 +2,9 @@
 // mofft_cuda.h.  Each registry entry is one compiled variant (precision, line
 // length, threads per line, lines per CTA, in-CTA radix chain).  The host
 // planner picks entries; the MEASURE planner times them.
+#include <atomic>
 #include <map>
+#include <memory>
 #include <tuple>
 #include <vector>
 
@@ -65,20 +67,55 @@ extern "C" size_t mofft_cuda_generic_smem(int precision_bits, int length,
                               : generic_smem<double>(length, lines, cols);
 }
 
-extern "C" int mofft_cuda_prepare_device(void) {
-  for (const Entry &e : registry()) {
-    size_t smem = e.desc.smem_bytes;
-    if (smem > 227 * 1024) smem = 227 * 1024;
-    cudaError_t err = cudaFuncSetAttribute(
-        e.func(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err == cudaSuccess && e.func_tail)
-      err = cudaFuncSetAttribute(e.func_tail(),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// Opts one registry kernel into its shared memory on the current device.
+static cudaError_t prepare_entry(int kernel) {
+  const auto &r = registry();
+  constexpr int kDevices = 64;
+  int device = 0;
+  const cudaError_t have = cudaGetDevice(&device);
+  if (have != cudaSuccess) return have;
+  if (device < 0 || device >= kDevices) return cudaErrorInvalidDevice;
+  static const std::unique_ptr<std::atomic<bool>[]> done(
+      new std::atomic<bool>[kDevices * r.size()]());
+  std::atomic<bool> &mine = done[(size_t)device * r.size() + (size_t)kernel];
+  if (mine.load(std::memory_order_acquire)) return cudaSuccess;
+  const Entry &e = r[kernel];
+  size_t smem = e.desc.smem_bytes;
+  if (smem > 227 * 1024) smem = 227 * 1024;
+  cudaError_t err =
+      cudaFuncSetAttribute(e.func(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err == cudaSuccess && e.func_tail)
+    err = cudaFuncSetAttribute(e.func_tail(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)smem);
+  if (err == cudaSuccess) mine.store(true, std::memory_order_release);
+  return err;
+}
+
+// Setting a kernel's attribute loads it, about 0.2 ms each, so a plan prepares the
+// kernels that its passes launch and not the whole registry: the first plan of a
+// process took 117 ms with all of them, 9 with its own.
+extern "C" int mofft_cuda_prepare_pass(int kernel, const mofft_pass_args *args) {
+  const auto &r = registry();
+  if (kernel < 0 || kernel >= (int)r.size() || !args) return (int)cudaErrorInvalidValue;
+  const mofft_kernel_desc &d = r[kernel].desc;
+  if (d.kind == MOFFT_KERNEL_GENERIC && d.bank == 0 && d.radices[0] <= 16) {
+    const cudaError_t err =
+        d.precision_bits == 32 ? rt_prepare_f32(args) : rt_prepare_f64(args);
+    if (err != cudaErrorNotSupported) return (int)err;
+  }
+  return (int)prepare_entry(kernel);
+}
+
+extern "C" int mofft_cuda_prepare_columns(int precision_bits) {
+  for (int i = 0; i < (int)registry().size(); ++i) {
+    const mofft_kernel_desc &d = registry()[i].desc;
+    if (d.precision_bits != precision_bits || d.bank != 0 ||
+        (d.kind != MOFFT_KERNEL_COLS && d.kind != MOFFT_KERNEL_GENERIC))
+      continue;
+    const cudaError_t err = prepare_entry(i);
     if (err != cudaSuccess) return (int)err;
   }
-  cudaError_t err = rt_prepare_f32();
-  if (err == cudaSuccess) err = rt_prepare_f64();
-  return (int)err;
+  return (int)(precision_bits == 32 ? rt_prepare_columns_f32() : rt_prepare_columns_f64());
 }
 
 extern "C" size_t mofft_cuda_kernel_aux_bytes(int kernel) {

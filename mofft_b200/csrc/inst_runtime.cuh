@@ -19,11 +19,17 @@ bool rt_pass_shape(const mofft_pass_args *p, RtShape *s) {
                   p->radix_count, line_units * p->batch, line_units, s);
 }
 
+inline int rt_mode(const mofft_pass_args *p, const RtShape &s) {
+  if (!p->generic_cols) return s.staged ? kRtStaged : kRtRows;
+  return p->ns_outer == 1 ? kRtColsHead : kRtColsTail;
+}
+
 // Smallest register class that holds the chain's largest radix, or the
 // several-butterfly kernels.
 template <typename T, int MODE>
 const void *rt_func(int max_radix, bool multi) {
-  if (multi) return reinterpret_cast<const void *>(&rt_kernel<T, MODE, 16, true>);
+  if constexpr (MODE != kRtStaged)   // one stage: one butterfly per thread
+    if (multi) return reinterpret_cast<const void *>(&rt_kernel<T, MODE, 16, true>);
   if (max_radix <= 8) return reinterpret_cast<const void *>(&rt_kernel<T, MODE, 8, false>);
   if (max_radix <= 11) return reinterpret_cast<const void *>(&rt_kernel<T, MODE, 11, false>);
   return reinterpret_cast<const void *>(&rt_kernel<T, MODE, 16, false>);
@@ -87,22 +93,35 @@ cudaError_t rt_launch(const mofft_pass_args *p, cudaStream_t stream) {
   const long long grid = cols ? ((long long)a.total_lines + s.lines - 1) / s.lines * p->batch
                               : (p->batch + s.lines - 1) / s.lines;
   if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  const int mode = cols ? (a.ns_outer == 1 ? kRtColsHead : kRtColsTail)
-                        : (s.staged ? kRtStaged : kRtRows);
-  const void *func = rt_func<T>(mode, s.max_radix, s.multi != 0);
+  const void *func = rt_func<T>(rt_mode(p, s), s.max_radix, s.multi != 0);
   return launch_pass(func, (unsigned)grid, s.threads, s.smem, a, p, stream);
 }
 
 template <typename T>
-cudaError_t rt_prepare() {
-  const int radix[] = {8, 11, 16, 16};
-  for (int i = 0; i < 4; ++i)
-    for (int mode = kRtRows; mode <= kRtColsTail; ++mode) {
-      const cudaError_t err =
-          cudaFuncSetAttribute(rt_func<T>(mode, radix[i], i == 3),
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-      if (err != cudaSuccess) return err;
-    }
+cudaError_t rt_opt_in(int mode, int max_radix, bool multi) {
+  return cudaFuncSetAttribute(rt_func<T>(mode, max_radix, multi),
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
+// The kernels that a pass of this shape launches: both forms, since the tile
+// depends on the launch's batch too (whether a tile fits does not).
+template <typename T>
+cudaError_t rt_prepare(const mofft_pass_args *p) {
+  RtShape s;
+  if (!rt_pass_shape<T>(p, &s)) return cudaErrorNotSupported;
+  const int mode = rt_mode(p, s);
+  const cudaError_t err = rt_opt_in<T>(mode, s.max_radix, false);
+  return err != cudaSuccess || s.staged ? err : rt_opt_in<T>(mode, s.max_radix, true);
+}
+
+template <typename T>
+cudaError_t rt_prepare_columns() {
+  for (int mode : {kRtColsHead, kRtColsTail})
+    for (int radix : {8, 11, 16})
+      for (bool multi : {false, true}) {
+        const cudaError_t err = rt_opt_in<T>(mode, radix, multi);
+        if (err != cudaSuccess) return err;
+      }
   return cudaSuccess;
 }
 

@@ -5,5 +5,6 @@ namespace mofft {
 cudaError_t rt_launch_f32(const mofft_pass_args *p, cudaStream_t s) {
   return rt_launch<float>(p, s);
 }
-cudaError_t rt_prepare_f32() { return rt_prepare<float>(); }
+cudaError_t rt_prepare_f32(const mofft_pass_args *p) { return rt_prepare<float>(p); }
+cudaError_t rt_prepare_columns_f32() { return rt_prepare_columns<float>(); }
 }  // namespace mofft

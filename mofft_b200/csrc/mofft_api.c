@@ -110,19 +110,6 @@ int mofft_device_family(uint32_t *family) {
   return 1;
 }
 
-/* Per-device one-time kernel attribute setup. */
-static atomic_int g_prepared[64];
-
-static int prepare_current_device(void) {
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess) return 0;
-  if (device < 0 || device >= 64) return 0;
-  if (atomic_load(&g_prepared[device]) == 1) return 1;
-  if (mofft_cuda_prepare_device() != 0) return 0;
-  atomic_store(&g_prepared[device], 1);
-  return 1;
-}
-
 /* ------------------------------------------------------------------------ */
 /* twiddles: exp(-2*pi*i*num/den) with exact octant reduction               */
 /* ------------------------------------------------------------------------ */
@@ -880,6 +867,19 @@ static mofft_status materialise_schedule(mofft_core *c) {
   size_t bytes = 0;
   for (int p = 0; p < c->sched.pass_count; ++p) {
     mofft_pass *ps = &c->sched.pass[p];
+    mofft_pass_args shape;
+    memset(&shape, 0, sizeof(shape));
+    shape.batch = (long long)c->batch;
+    shape.total = (long long)c->length;
+    shape.ns_outer = ps->ns_outer;
+    shape.generic_cols = c->sched.pass_count > 1;
+    shape.length = ps->length;
+    shape.radix_count = ps->radix_count;
+    memcpy(shape.radices, ps->radices, sizeof(shape.radices));
+    if (mofft_cuda_prepare_pass(ps->kernel, &shape) != 0) {
+      cudaGetLastError();
+      return MOFFT_UNSUPPORTED_HARDWARE;
+    }
     ps->tw_offset = bytes;
     bytes = align256(bytes + mofft_stage_table_entries(ps->radices, ps->radix_count) * cb + cb);
     ps->split_shift = 0;
@@ -1137,7 +1137,6 @@ mofft_status mofft_core_create_tuned(mofft_core **out, int precision_bits,
   if (distance == 0) distance = length;
   if (distance < length) return MOFFT_INVALID_ARGUMENT;
   if (batch > SIZE_MAX / distance / 16) return MOFFT_ALLOCATION_FAILURE;
-  if (!prepare_current_device()) return MOFFT_UNSUPPORTED_HARDWARE;
   mofft_core *c = (mofft_core *)calloc(1, sizeof(*c));
   if (!c) return MOFFT_ALLOCATION_FAILURE;
   pthread_mutex_init(&c->lock, NULL);

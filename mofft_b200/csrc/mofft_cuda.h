@@ -99,9 +99,12 @@ size_t mofft_cuda_generic_smem(int precision_bits, int length, int lines,
 int mofft_cuda_runtime_tile(int precision_bits, int cols, int length,
                             const int *chain, int count, long long line_units,
                             int *lines, int *threads, size_t *smem, int *ctas);
-/* Opt every kernel into its shared-memory size on the current device.
- * Returns a cudaError_t value (0 = success). */
-int mofft_cuda_prepare_device(void);
+/* Opt the kernels into their shared-memory size on the current device, before
+ * the first launch: those that a pass launches whatever its batch (args: the
+ * pass's shape, no pointers), or every one of bank 0 that a pass of a
+ * multi-pass transform may launch.  Return a cudaError_t value (0 = success). */
+int mofft_cuda_prepare_pass(int kernel, const mofft_pass_args *args);
+int mofft_cuda_prepare_columns(int precision_bits);
 /* Bytes of the B operand tiles of a tensor-core precision form (0 if the
  * form has no tensor-core kernel), and their host-side construction from the
  * 16-point forward DFT matrix fr + i fi (row-major F[k][r]). */

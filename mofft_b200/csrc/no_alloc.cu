@@ -83,7 +83,7 @@ int ceil_log2(unsigned long long x) {
 size_t round32(size_t x) { return (x + 31) & ~size_t(31); }
 
 // Resolve (once per device, with that device current) the device address of
-// g_fixed_scratch and opt the kernels into their shared memory sizes.
+// g_fixed_scratch and opt the column kernels into their shared memory sizes.
 mofft_status scratch_address(int device, float2 **out) {
   if (device < 0 || device >= kMaxDevices) return MOFFT_UNSUPPORTED_HARDWARE;
   std::lock_guard<std::mutex> lock(g_setup_mutex);
@@ -93,7 +93,7 @@ mofft_status scratch_address(int device, float2 **out) {
       cudaGetLastError();
       return MOFFT_INTERNAL_ERROR;
     }
-    if (mofft_cuda_prepare_device() != 0) {
+    if (mofft_cuda_prepare_columns(32) != 0) {
       cudaGetLastError();
       return MOFFT_INTERNAL_ERROR;
     }
