@@ -639,24 +639,40 @@ static void collect_divisors(long long n, long long lo, long long hi,
 }
 
 static int model_chain(int precision_bits, unsigned bank, size_t length, int *chain,
-                       int capacity, int one_pass);
+                       int capacity, int one_pass, mofft_schedule *split);
 
 /* Analytical PRETUNED chain for a whole transform of `length`. */
 int mofft_model_chain(int precision_bits, unsigned bank, size_t length,
                       int *chain, int capacity) {
-  return model_chain(precision_bits, bank, length, chain, capacity, 1);
+  return model_chain(precision_bits, bank, length, chain, capacity, 1, NULL);
 }
 
 /* The best chain of two or more passes (callers that need the intermediate
  * array of a multi-pass schedule even where one pass exists). */
 int mofft_model_chain_multipass(int precision_bits, unsigned bank, size_t length,
                                 int *chain, int capacity) {
-  return model_chain(precision_bits, bank, length, chain, capacity, 0);
+  return model_chain(precision_bits, bank, length, chain, capacity, 0, NULL);
+}
+
+/* The best split of a length that only the runtime-chain kernels run in one pass
+ * (runs_in_one_pass: that schedule), for callers that need compiled kernels or an
+ * intermediate array; grouped as it is, since its chain would regroup into the
+ * one pass.  Shorter lengths, which the ping-pong kernel's tile holds too, have
+ * no split here.  Returns the chain's stages or 0. */
+int mofft_model_split(int precision_bits, size_t length, const mofft_schedule *runs_in_one_pass,
+                      int *chain, int capacity, mofft_schedule *split) {
+  if (runs_in_one_pass->pass_count != 1 ||
+      runs_in_one_pass->pass[0].kind != MOFFT_KERNEL_GENERIC ||
+      mofft_cuda_generic_smem(precision_bits, (int)length, 1, 0) <= SMEM_LIMIT)
+    return 0;
+  const int count = model_chain(precision_bits, 0, length, chain, capacity, 0, split);
+  return count > 0 ? count : 0;
 }
 
 typedef struct {
   int chain[MOFFT_MAX_STAGES];
   int count;
+  int cuts[MOFFT_MAX_PASSES];
   group_score score;
   double seconds;
 } ranked_split;
@@ -717,7 +733,7 @@ static int split_less(const ranked_split *a, const ranked_split *b) {
 }
 
 static int model_chain(int precision_bits, unsigned bank, size_t length, int *chain,
-                       int capacity, int one_pass) {
+                       int capacity, int one_pass, mofft_schedule *split) {
   mofft_schedule sched;
   /* one pass */
   int count = one_pass ? preferred_chain(precision_bits, bank, MOFFT_KERNEL_ROWS,
@@ -760,17 +776,16 @@ static int model_chain(int precision_bits, unsigned bank, size_t length, int *ch
         c.count = 0;
         long long ns = 1;
         int ok = 1;
-        int cuts[MOFFT_MAX_PASSES];
         for (int p = 0; p < passes && ok; ++p) {
           if (L[p] < 2 || L[p] > (1 << 16)) { ok = 0; break; }
           const int k = preferred_chain(precision_bits, bank, MOFFT_KERNEL_COLS, L[p], n, ns,
                                         memo, c.chain + c.count, MOFFT_MAX_STAGES - c.count);
           if (k <= 0) { ok = 0; break; }
           c.count += k;
-          if (p < passes - 1) cuts[p] = c.count;
+          if (p < passes - 1) c.cuts[p] = c.count;
           ns *= L[p];
         }
-        if (!ok || !try_split(precision_bits, bank, c.chain, c.count, cuts, passes, n, NULL,
+        if (!ok || !try_split(precision_bits, bank, c.chain, c.count, c.cuts, passes, n, NULL,
                               &sched, &c.score))
           continue;
         c.seconds = split_cost(precision_bits, bank, (size_t)n, model_batch, &sched,
@@ -785,6 +800,14 @@ static int model_chain(int precision_bits, unsigned bank, size_t length, int *ch
     }
   }
   free(memo);
+  if (split) {
+    group_score score;
+    if (nkept == 0 || !try_split(precision_bits, bank, kept[0].chain, kept[0].count,
+                                 kept[0].cuts, kept[0].score.passes, n, NULL, split, &score))
+      return -1;
+    memcpy(chain, kept[0].chain, (size_t)kept[0].count * sizeof(int));
+    return kept[0].count;
+  }
   int best = -1;
   for (int i = 0; i < nkept; ++i) {
     if (!mofft_group_chain(precision_bits, bank, kept[i].chain, kept[i].count, n, &sched))

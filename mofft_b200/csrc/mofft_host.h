@@ -30,6 +30,8 @@ int mofft_model_chain(int precision_bits, unsigned bank, size_t length,
 /* The best chain of two or more passes for `length` (-1 if none). */
 int mofft_model_chain_multipass(int precision_bits, unsigned bank, size_t length,
                                 int *chain, int capacity);
+int mofft_model_split(int precision_bits, size_t length, const mofft_schedule *runs_in_one_pass,
+                      int *chain, int capacity, mofft_schedule *split);
 
 mofft_status mofft_core_create(mofft_core **out, int precision_bits,
                                size_t length, size_t batch, size_t distance,

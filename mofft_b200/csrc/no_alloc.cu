@@ -157,6 +157,10 @@ extern "C" mofft_status mofft_execute_fixed_scratch_f32(
       if (count <= 0 || !mofft_group_chain(32, 0, chain, count, (long long)length, &sched))
         return MOFFT_UNSUPPORTED_SIZE;
     }
+    // So has one that only the runtime-chain kernels compute in one pass
+    // (14112 to 15360 points).
+    mofft_schedule split;
+    if (mofft_model_split(32, length, &sched, chain, MOFFT_MAX_STAGES, &split) > 0) sched = split;
   }
   if (sched.pass_count != 2) return MOFFT_UNSUPPORTED_SIZE;
 

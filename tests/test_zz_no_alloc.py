@@ -125,3 +125,23 @@ def test_limits_are_rejected():
     assert lib.mofft_execute_fixed_scratch_f32(host.ctypes.data, host.ctypes.data, 1 << 16, 1,
                                                m.FORWARD, None) == m.Status.INVALID_ARGUMENT
     assert LIMIT == 1 << 22
+
+
+@pytest.mark.parametrize("n", [14112, 14175, 14336, 14400, 14580, 15000, 15360])
+def test_lengths_beyond_the_ping_pong_tile(n):
+    """Lengths that only the runtime-chain kernels compute in one pass keep
+    their two-pass schedule here."""
+    import torch
+    lib = m.load()
+    _bind(lib)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.view_as_complex(torch.rand((3, n, 2), generator=gen, device="cuda") * 2 - 1)
+    y = torch.empty_like(x)
+    torch.cuda.synchronize()
+    for direction in (m.FORWARD, m.BACKWARD):
+        assert _fixed(lib, x, y, n, 3, direction) == m.Status.SUCCESS
+        torch.cuda.synchronize()
+        ref = _oracle_rows(x, direction, [0, 1, 2])
+        assert rel_l2(y.cpu().numpy(), ref) <= fp32_tol(n)
+    # the longest one of the ping-pong tile runs in one pass, as before
+    assert _fixed(lib, x, y, 14040, 1, m.FORWARD) == m.Status.UNSUPPORTED_SIZE
