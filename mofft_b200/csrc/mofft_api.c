@@ -1147,6 +1147,27 @@ mofft_status mofft_core_create_pretuned(mofft_core **out, int precision_bits, si
                                  tuned > 0 ? preferred : NULL);
 }
 
+/* An out-of-place plan for callers that launch through pointer tables, which the
+ * runtime-chain kernels do not take: where those run the length in one pass and
+ * compiled kernels run it in two (FP32 15360, FP64 7680), the compiled ones. */
+mofft_status mofft_core_create_for_tables(mofft_core **out, int precision_bits, size_t length,
+                                          size_t batch, size_t distance,
+                                          mofft_direction direction) {
+  mofft_status st = mofft_core_create_pretuned(out, precision_bits, length, batch, distance,
+                                               direction, MOFFT_OUT_OF_PLACE);
+  if (st != MOFFT_SUCCESS) return st;
+  int chain[MOFFT_MAX_STAGES], kernels[MOFFT_MAX_PASSES];
+  mofft_schedule split;
+  const int count = mofft_model_split(precision_bits, length, &(*out)->sched, chain,
+                                      MOFFT_MAX_STAGES, &split);
+  if (count <= 0 || generic_passes(&split) > 0) return MOFFT_SUCCESS;
+  for (int p = 0; p < MOFFT_MAX_PASSES; ++p)
+    kernels[p] = p < split.pass_count ? split.pass[p].kernel : -1;
+  mofft_core_destroy(*out);
+  return mofft_core_create_tuned(out, precision_bits, length, batch, distance, direction,
+                                 MOFFT_OUT_OF_PLACE, chain, count, kernels);
+}
+
 mofft_status mofft_core_create_tuned(mofft_core **out, int precision_bits,
                                      size_t length, size_t batch,
                                      size_t distance, mofft_direction direction,

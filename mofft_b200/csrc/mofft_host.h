@@ -62,6 +62,10 @@ mofft_status mofft_core_enqueue_tables(const mofft_core *c, const void *const *c
 mofft_status mofft_core_create_pretuned(mofft_core **out, int precision_bits, size_t length,
                                         size_t batch, size_t distance,
                                         mofft_direction direction, mofft_placement placement);
+/* The same for launches through pointer tables. */
+mofft_status mofft_core_create_for_tables(mofft_core **out, int precision_bits, size_t length,
+                                          size_t batch, size_t distance,
+                                          mofft_direction direction);
 mofft_status mofft_core_enqueue_indirect(const mofft_core *c, const void *const *in_table,
                                          void *const *out_table, long long batch,
                                          void *stream);

@@ -329,8 +329,8 @@ static mofft_status ragged_fail(mofft_ragged_plan *p, mofft_status st) {
 // (at most two passes of specialised kernels).
 static mofft_core *group_core(long long n, mofft_direction direction, long long transforms) {
   mofft_core *c = nullptr;
-  if (mofft_core_create_pretuned(&c, 32, (size_t)n, (size_t)transforms, (size_t)n, direction,
-                                 MOFFT_OUT_OF_PLACE) != MOFFT_SUCCESS)
+  if (mofft_core_create_for_tables(&c, 32, (size_t)n, (size_t)transforms, (size_t)n,
+                                   direction) != MOFFT_SUCCESS)
     return nullptr;
   bool ok = c->sched.pass_count >= 1 && c->sched.pass_count <= 2;
   for (int q = 0; ok && q < c->sched.pass_count; ++q)

@@ -121,8 +121,7 @@ mofft_core *plan_for(mofft_server *S, const mofft_request &r, mofft_status *st) 
   // one, else the model's, where it has more passes than a pointer-table group
   // runs (two)
   mofft_core *c = nullptr;
-  *st = mofft_core_create_pretuned(&c, r.precision_bits, r.length, 1, 0, r.direction,
-                                   MOFFT_OUT_OF_PLACE);
+  *st = mofft_core_create_for_tables(&c, r.precision_bits, r.length, 1, 0, r.direction);
   if (*st == MOFFT_SUCCESS && c->sched.pass_count > 2) {
     mofft_core_destroy(c);
     c = nullptr;

@@ -156,3 +156,20 @@ def test_long_items_run_as_tuned_groups():
         ref = oracle.fft_ld(x.cpu().numpy().astype(np.complex128), d)
         assert rel_l2(out.cpu().numpy(), ref) <= fp32_tol(n), n
     plan.destroy()
+
+
+def test_a_length_of_one_runtime_pass():
+    """15360 points run in one pass of a kernel that takes no pointer tables;
+    in a ragged batch they run as two passes of compiled kernels."""
+    import torch
+    spec = [(15360, 2, -1), (1024, 3, 1), (15360, 1, 1), (15360, 4, -1)]
+    items = make_items(spec, inplace=lambda k: k == 3)
+    plan = m.RaggedPlan([(a, b, d) for a, b, d, _ in items])
+    plan.execute()
+    torch.cuda.synchronize()
+    assert plan.status() == 0
+    for _, out, direction, orig in items:
+        x = orig.cpu().numpy()
+        ref = oracle.fft_ld(x.astype(np.complex128), direction)
+        assert rel_l2(out.cpu().numpy(), ref) <= fp32_tol(x.shape[-1])
+    plan.destroy()

@@ -193,3 +193,24 @@ def test_lengths_on_runtime_stage_kernels():
         ref = oracle.fft_ld(x.cpu().numpy().astype(np.complex128), -1)
         assert rel_l2(y.cpu().numpy(), ref) <= (fp32_tol(n) if bits == 32 else fp64_tol(n))
     srv.destroy()
+
+
+@pytest.mark.parametrize("n,bits", [(15360, 32), (7680, 64)])
+def test_lengths_of_one_runtime_pass_coalesce(n, bits):
+    """Their one-pass kernel takes no pointer tables; requests run as groups of
+    two compiled passes instead of a launch each."""
+    import torch
+    ins = [_tensor(1, n, bits, 300 + k) for k in range(64)]
+    outs = [torch.empty_like(x) for x in ins]
+    torch.cuda.synchronize()
+    srv = m.Server(streams=1)
+    before = m.launch_count()
+    for x, out in zip(ins, outs):
+        srv.submit(n, 1, -1, bits, x.data_ptr(), out.data_ptr())
+    srv.drain()
+    assert m.launch_count() - before < len(ins)
+    srv.destroy()
+    got = torch.cat(outs).cpu().numpy()
+    ref = oracle.fft_ld(torch.cat(ins).cpu().numpy().astype(np.complex128), -1)
+    tol = fp32_tol(n) if bits == 32 else fp64_tol(n)
+    assert rel_l2(got, ref) <= tol
