@@ -1,0 +1,82 @@
+"""Passes start while the stream's previous kernel drains: chains of dependent
+executes of different kernel kinds without a synchronize in between give the
+bits that the same executes give one at a time, on a stream, across streams
+joined by events and in a captured graph."""
+from __future__ import annotations
+
+import pytest
+
+import mofft_b200 as m
+from tests.conftest import cuda_available
+
+pytestmark = [pytest.mark.gpu,
+              pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")]
+
+POINTS = 2 * 65536 * 27
+# (length, bank): a two-line, a pair, a runtime and a ping-pong kernel of one
+# pass, compiled and runtime column passes, two of them with a workspace
+STEPS = [(512, 0), (4096, 0), (3456, 0), (768, 1), (65536, 0), (221184, 0), (256, 0), (1769472, 0)]
+
+
+def plans(stream, bits):
+    made = []
+    for k, (n, bank) in enumerate(STEPS):
+        p = m.Plan.create(n, m.FORWARD if k % 2 else m.BACKWARD, m.IN_PLACE, bits=bits,
+                          batch=POINTS // n)
+        if bank:
+            p.set_kernel_bank(bank)
+        p.set_stream(stream)
+        made.append(p)
+    return made
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+def test_chains_of_dependent_passes(bits):
+    import torch
+    assert all(POINTS % n == 0 for n, _ in STEPS)
+    dtype = torch.complex64 if bits == 32 else torch.complex128
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    ops = plans(a.cuda_stream, bits)
+    other = plans(b.cuda_stream, bits)
+    g = torch.Generator(device="cuda").manual_seed(bits)
+    real = torch.float32 if bits == 32 else torch.float64
+    x = torch.view_as_complex(torch.rand((POINTS, 2), generator=g, device="cuda",
+                                         dtype=real) * 2 - 1).to(dtype)
+
+    ref = x.clone()
+    torch.cuda.synchronize()
+    for p in ops:                                   # one at a time
+        p.execute(ref)
+        torch.cuda.synchronize()
+
+    for _ in range(3):                              # back to back on one stream
+        y = x.clone()
+        torch.cuda.synchronize()
+        for p in ops:
+            p.execute(y)
+        torch.cuda.synchronize()
+        assert torch.equal(torch.view_as_real(y), torch.view_as_real(ref))
+
+    y = x.clone()                                   # two streams, joined by events
+    torch.cuda.synchronize()
+    for k in range(len(STEPS)):
+        here, there = (a, b) if k % 2 else (b, a)
+        (ops if here is a else other)[k].execute(y)
+        there.wait_stream(here)
+    torch.cuda.synchronize()
+    assert torch.equal(torch.view_as_real(y), torch.view_as_real(ref))
+
+    y = x.clone()                                   # captured, replayed twice
+    src = x.clone()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=a):
+        y.copy_(src)
+        for p in ops:
+            p.execute(y)
+    for _ in range(2):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(torch.view_as_real(y), torch.view_as_real(ref))
+    for p in ops + other:
+        p.destroy()

@@ -480,3 +480,24 @@ def test_planning_stays_short(n, bits):
         m.schedule_preview(n, bits)
         best = min(best, time.perf_counter() - t)
     assert best < 3.5e-3
+
+
+def test_long_smooth_lengths_of_every_prime():
+    """Every 13-smooth length between 2^14 and 2^20, all primes up to 13 among
+    their factors, splits into two or three passes of tiles that fit."""
+    def smooth(n):
+        for p in (2, 3, 5, 7, 11, 13):
+            while n % p == 0:
+                n //= p
+        return n == 1
+
+    lengths = [n for n in range(1 << 14, 1 << 20) if smooth(n)]
+    for p in (2, 3, 5, 7, 11, 13):
+        assert sum(n % p == 0 for n in lengths) > 500
+    for bits in (32, 64):
+        for n in lengths:
+            s = m.schedule_preview(n, bits)
+            assert int(np.prod(s["radices"])) == n and int(np.prod(s["lengths"])) == n
+            assert s["pass_count"] <= 3
+            assert all(0 < b <= 227 * 1024 for b in s["smem_bytes"])
+            assert all(2 <= r <= 16 or r in (32, 64) for r in s["radices"])
