@@ -6,11 +6,12 @@
 // butterflies do not divide evenly) and as many registers.  Here the odd factor
 // sits inside a radix of 10 or 12 (or a radix of its own with two to four
 // butterflies a thread) behind a radix-16 or radix-8 stage: at most 16 points
-// and 32 to 48 registers a thread in FP32 (64 to 70 before), up to 108 in FP64.  A power of two first also
-// makes the pad every 16 pairs free of bank conflicts (a bank simulation:
-// 1.0-1.2 wavefronts per access against 1.35-1.9).  Lengths below 400 used to
-// copy their lines through shared memory on both sides; reading and writing
-// runs of L / radix points directly takes less, down to runs of 48 bytes.
+// and 32 to 48 registers a thread in FP32 (64 to 70 before), up to 108 in FP64.
+// A power of two first also makes the pad every 16 pairs free of bank conflicts
+// (a bank simulation: 1.0-1.2 wavefronts per access against 1.35-1.9).  Lengths
+// below 400 used to copy their lines through shared memory on both sides;
+// reading and writing runs of L / radix points directly takes less, down to
+// runs of 48 bytes.
 //
 // us per 2^25 FP32 / 2^24 FP64 points (copy floor 82), before -> now: FP32 64
 // 93 -> 85, 80 122 -> 99, 160 130 -> 86, 192 115 -> 83, 320 133 -> 107, 384

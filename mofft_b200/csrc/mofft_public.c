@@ -121,8 +121,8 @@ static mofft_status create_with_options(mofft_core **out, int precision_bits,
    * not (unless the caller insists on wisdom).  Out of place the plan then
    * takes the two-pass schedule the wisdom keeps beside the three-pass one;
    * lengths without one (FP32 2^24, FP64 2^23 and 2^24: 4096-point columns in
-   * runs of 32 bytes take 1.3 times as long as three narrow passes, 216
-   * against 163 us) run the three passes with a workspace. */
+   * runs of 32 bytes take 1.5 times as long as three narrow passes, FP32 2^24
+   * 216 against 148 us) run the three passes with a workspace. */
   if (wisdom && !(options.flags & MOFFT_PLAN_STRICT_WISDOM)) {
     int tuned_passes = 0;
     while (tuned_passes < MOFFT_MAX_PASSES && preferred[tuned_passes] >= 0) ++tuned_passes;

@@ -2,13 +2,13 @@
 // launch argument, for the 13-smooth lengths without a compiled instance.
 //
 // A tile is `lines` lines of L points (ROWS: whole transforms; COLS: adjacent
-// super-butterflies of a multi-pass transform).  A thread runs at most one
-// butterfly per stage: it gathers R values into registers, multiplies the
-// stage twiddles, runs the straight-line radix-R codelet and, once every
-// thread of the CTA has read, scatters into the same shared-memory tile.  So
-// a tile needs one copy of its points (the ping-pong form this replaces kept
-// four component arrays), and every value crosses shared memory as one
-// {re, im} pair.
+// super-butterflies of a multi-pass transform).  A thread runs one butterfly
+// per stage, or in the several-butterfly form as many as hold 16 points (eight
+// of radix 2): it gathers R values each into registers, multiplies the stage
+// twiddles, runs the straight-line radix-R codelet and, once every thread of
+// the CTA has read, scatters into the same shared-memory tile.  So a tile needs
+// one copy of its points (the ping-pong form this replaces kept four component
+// arrays), and every value crosses shared memory as one {re, im} pair.
 //
 // Addresses.  With Ns the product of the radices applied so far, stage
 // (R, Ns) scatters butterfly j to (j / Ns) Ns R + (j mod Ns) + k Ns and the

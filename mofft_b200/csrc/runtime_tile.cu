@@ -9,8 +9,7 @@
 namespace mofft {
 
 static const size_t kSmemLimit = 227 * 1024;
-static const int kSms = 148;
-
+static const int kSms = 148;   // of the B200, the only target
 
 // Pad pairs behind each block of ns * radix points of an exchange.  First
 // exchange: an even radix scatters at an even stride, one pad makes it odd.

@@ -12,13 +12,13 @@
 // {reA, reB, imA, imB}, the layout of the FP64 pair tiles.
 //
 // Measured against the one-line instances (us, 2^26 points / 2^21 points in
-// L2): 64 164 -> 154 / 8.1 -> 7.9, 128 177 -> 162 / 10.0 -> 8.9, 256 158 -> 157
-// / 9.4 -> 7.7, 320 209 -> 177, 384 184 -> 156, 512 169 -> 156 / 9.1 -> 8.8,
-// 1280 183 -> 169, 1536 168 -> 160; under sustained load 256 174 -> 164, 512
-// 196 -> 182.  Not built where one line already takes half an SM's tile or
-// registers: a pair halves the resident CTAs, whose barriers then show (4096
-// 170 -> 181, 8192 223 -> 291, 3072 171 -> 189, 2560 177 -> 205), nor where it
-// loses in L2 (160, 192, 640, 768, 1024, 2048).
+// L2): 48 198 -> 187 / 7.3 -> 7.0, 64 163 -> 155 / 5.8 -> 5.5, 96 186 -> 177 / 7.4
+// -> 7.9, 128 177 -> 161 / 6.0 -> 5.6, 256 158 -> 157 / 6.2 -> 5.7, 320 208 -> 176 /
+// 7.9 -> 7.0, 384 184 -> 164 / 7.1 -> 6.7, 512 169 -> 156 / 7.4 -> 6.9, 1280 183 ->
+// 174 / 7.5 -> 7.3, 1536 172 -> 163 / 7.1 -> 6.7.  Not built where one line
+// already takes half an SM's tile or registers: a pair halves the resident CTAs,
+// whose barriers then show (4096 170 -> 181, 8192 223 -> 291, 3072 171 -> 189,
+// 2560 177 -> 205), nor where it loses in L2 (160, 192, 640, 768, 1024, 2048).
 //
 // Every stage twiddle is looked up.  Forming powers above w^3 as products took
 // 1 % less time (5 % at 48 and 384: 95 -> 91, 85 -> 81 us of 2^25 points) and
@@ -295,14 +295,13 @@ twin_kernel(const RowsArgs<float> args) {
 // Lines of 320-512 points are bound by their tiles: 8 lines on 256 threads move
 // 64-byte runs, and 16 lines of the one-line form take 512 threads at 64
 // registers.  Two lines a thread give 16 lines, 128-byte runs, on 256 threads
-// at 110 registers with two CTAs per SM.  us per 2^25 points, 8 lines -> 16
+// at 116 registers with two CTAs per SM.  us per 2^25 points, 8 lines -> 16
 // lines one a thread -> 16 lines two a thread: 512 x 160 224 -> 211 -> 199, 512
 // x 192 220 -> 206 -> 194, 256 x 512 209 -> 209 -> 199, 512 x 1024 261 -> 248
 // -> 237; 512 x 512 239 -> 218 (256 x 1024 takes 220); as the narrow side of
 // 327680 and 393216, 320 and 384 points take
-// 279 -> 252 and 260 -> 247.  In L2 (2^21 points) 98304 18.6 -> 15.7, 131072
-// 17.6 -> 15.6.  One transform alone, with half the CTAs, takes up to 1.2 us
-// longer (131072 7.8 -> 9.0).  Not built for 64-256 points, whose one-line
+// 279 -> 254 and 260 -> 249.  In L2 (2^21 points) 131072 16.1 -> 14.1; one
+// transform alone, with half the CTAs, 8.4 -> 7.9.  Not built for 64-256 points, whose one-line
 // tiles already move 128-byte runs (256 x 256 184 -> 187, 64 x 64 170 -> 168),
 // nor for 640-2048 points, whose 16-line tiles leave one CTA per SM (512 x
 // 1024 237 -> 245).
