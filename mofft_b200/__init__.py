@@ -14,6 +14,7 @@ from __future__ import annotations
 import ctypes
 import enum
 import os
+import threading
 from pathlib import Path
 from typing import Optional, Sequence
 
@@ -336,6 +337,7 @@ class Plan:
         self._s = "f32" if bits == 32 else "f64"
         self._lib = load()
         self._execute = self._fn("execute")
+        self._stream: Optional[int] = None
 
     def _fn(self, name: str):
         return getattr(self._lib, f"mofft_{name}_{self._s}")
@@ -385,6 +387,7 @@ class Plan:
 
     def set_stream(self, stream_handle: Optional[int]) -> None:
         check(self._fn("plan_set_stream")(self._h, stream_handle or None), "set_stream")
+        self._stream = stream_handle or None
 
     def set_kernel_bank(self, bank: int) -> None:
         check(self._fn("plan_set_kernel_bank")(self._h, bank), "set_kernel_bank")
@@ -554,7 +557,9 @@ def fft(x, direction: int = FORWARD, *, inplace: bool = False):
 
     Runs in the order of torch's current stream.  On the default stream the
     call returns after the transform has completed; on any other stream it
-    enqueues and returns."""
+    enqueues and returns.  Can be captured into a graph once the shape has run;
+    where it takes a workspace, replays must not overlap calls of that shape on
+    the stream that ran it."""
     import torch
     if not x.is_cuda:
         raise ValueError("fft() takes a CUDA tensor; use Plan for host arrays")
@@ -568,13 +573,15 @@ def fft(x, direction: int = FORWARD, *, inplace: bool = False):
     device = x.get_device()
     current = torch.cuda.current_stream(device)
     stream = current.cuda_stream or _LEGACY_STREAM
-    plan = _plan_cache_get(n, batch, direction, inplace, bits, device, stream)
-    plan.execute(x, out)
-    if stream == _LEGACY_STREAM:
-        if bits == 32:
+    plan, lock = _plan_cache_get((n, batch, direction, inplace, bits, device), stream)
+    with lock:
+        if plan._stream != stream:
+            plan.set_stream(stream)
+        plan.execute(x, out)
+        if stream == _LEGACY_STREAM and bits == 32:
             plan.check_status()
-        else:  # no FP64 kernel keeps a status
-            current.synchronize()
+    if stream == _LEGACY_STREAM and bits == 64:  # no FP64 kernel keeps a status
+        current.synchronize()
     return out
 
 
@@ -586,16 +593,23 @@ _LEGACY_STREAM = 1
 _PLAN_CACHE: dict = {}
 
 
-def _plan_cache_get(n, batch, direction, inplace, bits, device, stream):
-    """The plan of a shape on a stream.  A plan stays on the stream it was made
-    for: plans of several passes may own a workspace, which calls on one
-    stream use in turn and calls on two streams would overwrite for each
-    other."""
-    key = (n, batch, direction, inplace, bits, device, stream)
-    plan = _PLAN_CACHE.get(key)
-    if plan is None:
-        plan = Plan.create(n, direction, IN_PLACE if inplace else OUT_OF_PLACE,
-                           bits=bits, batch=batch)
-        plan.set_stream(stream)
-        plan = _PLAN_CACHE.setdefault(key, plan)  # another thread's may be first
-    return plan
+def _plan_cache_get(shape, stream):
+    """A shape's plan and the lock under which it runs.  All streams share a plan
+    without a workspace; one with a workspace (several passes) belongs to a
+    stream, whose calls use the workspace in turn where two streams would
+    overwrite it for each other."""
+    entry = _PLAN_CACHE.get(shape) or _PLAN_CACHE.get(shape + (stream,))
+    if entry is not None:
+        return entry
+    import torch
+    if torch.cuda.is_current_stream_capturing():
+        # nothing can be allocated here: the plan of another stream, which the
+        # graph's replays then share with that stream's calls
+        for key, other in list(_PLAN_CACHE.items()):
+            if key[:-1] == shape:
+                return other
+    n, batch, direction, inplace, bits, _ = shape
+    plan = Plan.create(n, direction, IN_PLACE if inplace else OUT_OF_PLACE,
+                       bits=bits, batch=batch)
+    key = shape + (stream,) if plan.schedule()["workspace_bytes"] else shape
+    return _PLAN_CACHE.setdefault(key, (plan, threading.Lock()))

@@ -34,6 +34,7 @@ class FakeTensor:
 class FakePlan:
     """Records which stream it runs on, and the waits for it."""
     made: list = []
+    workspace = 0
 
     def __init__(self):
         self._stream, self.log = None, []
@@ -48,12 +49,17 @@ class FakePlan:
     def check_status(self):
         self.log.append(("wait", self._stream))
 
+    def schedule(self):
+        return {"workspace_bytes": FakePlan.workspace}
+
 
 @pytest.fixture
 def fakes(monkeypatch):
     """fft() on fake tensors, plans and streams; yields the stream's setter."""
     import torch
     FakePlan.made = []
+    monkeypatch.setattr(FakePlan, "workspace", 0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     monkeypatch.setattr(m, "_PLAN_CACHE", {})
     monkeypatch.setattr(m.Plan, "create", lambda *a, **k: FakePlan())
     monkeypatch.setattr(torch, "empty_like", lambda x: x)
@@ -79,23 +85,47 @@ def test_default_stream_keeps_its_order(fakes, bits):
     assert plan.log[1:] == ([("wait", 1)] if bits == 32 else []) and waits == [0] * (bits == 64)
 
 
-def test_streams_do_not_share_a_plan(fakes):
-    """A plan may own a workspace: no plan runs on two streams, and a stream's
-    second call finds its plan again."""
+@pytest.mark.parametrize("workspace", [0, 1 << 20])
+def test_streams_share_no_workspace(fakes, monkeypatch, workspace):
+    """A plan with a workspace runs on one stream only; one without runs on
+    each call's stream.  A stream's second call finds its plan again."""
     import torch
+    monkeypatch.setattr(FakePlan, "workspace", workspace)
     x = FakeTensor(65536, torch.complex64)
     for handle in (7, 9, 0, 7, 9, 0):
         fakes(handle)
         m.fft(x, inplace=True)
     ran = [[s for what, s in p.log if what == "run"] for p in FakePlan.made]
-    assert ran == [[7, 7], [9, 9], [1, 1]]
+    assert ran == ([[7, 7], [9, 9], [1, 1]] if workspace else [[7, 9, 1, 7, 9, 1]])
 
 
-def test_threads_do_not_move_each_others_stream(fakes, monkeypatch):
+@pytest.mark.parametrize("workspace", [0, 1 << 20])
+def test_capture_makes_no_plan(fakes, monkeypatch, workspace):
+    """A capture runs on a stream of its own and cannot allocate: it takes the
+    plan that the shape's earlier call made, and leaves that call's stream its
+    plan."""
+    import torch
+    monkeypatch.setattr(FakePlan, "workspace", workspace)
+    x = FakeTensor(65536, torch.complex64)
+    fakes(7)
+    m.fft(x, inplace=True)
+    fakes(9)
+    with monkeypatch.context() as patch:
+        patch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+        m.fft(x, inplace=True)
+    fakes(7)
+    m.fft(x, inplace=True)
+    (plan,) = FakePlan.made
+    assert [s for _, s in plan.log] == [7, 9, 7]
+
+
+@pytest.mark.parametrize("workspace", [0, 1 << 20])
+def test_threads_do_not_move_each_others_stream(fakes, monkeypatch, workspace):
     """Two threads on two streams, the second calling while the first one is
     inside its call: each transform runs on its own thread's stream."""
     import threading
     import torch
+    monkeypatch.setattr(FakePlan, "workspace", workspace)
     local = threading.local()
     monkeypatch.setattr(torch.cuda, "current_stream",
                         lambda device=None: types.SimpleNamespace(cuda_stream=local.handle))
@@ -107,7 +137,7 @@ def test_threads_do_not_move_each_others_stream(fakes, monkeypatch):
         with lock:
             seen.append((local.handle, self._stream))
     monkeypatch.setattr(FakePlan, "execute", execute)
-    real_set, turn = FakePlan.set_stream, threading.Barrier(2, timeout=2)
+    real_set, turn = FakePlan.set_stream, threading.Barrier(2, timeout=0.2)
 
     def set_stream(self, stream):
         real_set(self, stream)
@@ -193,3 +223,32 @@ def test_streams_with_a_workspace(n, batch, bits, inplace):
                 err = torch.linalg.vector_norm(y - ref) / torch.linalg.vector_norm(ref)
                 # the same kernels on the same input; in place may run another schedule
                 assert float(err) <= (fp32_tol(n) if bits == 32 else fp64_tol(n))
+
+
+@pytest.mark.gpu
+@needs_gpu
+@pytest.mark.parametrize("n,batch,bits,inplace", [(1024, 64, 32, False), (65536, 8, 32, True),
+                                                  (3375, 5, 64, False), (50625, 3, 64, True)])
+def test_capture_after_a_warm_up(n, batch, bits, inplace):
+    """The shape runs once on a side stream, then fft() is captured on the
+    graph's own stream and replayed."""
+    import torch
+    dtype = np.complex64 if bits == 32 else np.complex128
+    host = oracle.uniform(n * batch, seed=n, dtype=dtype).reshape(batch, n)
+    src = torch.from_numpy(host).cuda()
+    x = src.clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        m.fft(x.clone(), inplace=inplace)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x.copy_(src)
+        y = m.fft(x, inplace=inplace)
+    for _ in range(2):
+        y.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    ref = oracle.fft_ld(host.astype(np.complex128), -1)
+    assert rel_l2(y.cpu().numpy(), ref) <= (fp32_tol(n) if bits == 32 else fp64_tol(n))
