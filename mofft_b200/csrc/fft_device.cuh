@@ -1309,7 +1309,7 @@ struct GenericArgs {
 
 template <typename T, int R, int BANK>
 __device__ __forceinline__ void generic_butterfly(
-    const GenericArgs<T>& a, const T* __restrict__ sre_src,
+    const GenericArgs<T>& a, const cplx_t<T>* in, const T* __restrict__ sre_src,
     const T* __restrict__ sim_src, T* __restrict__ sre_dst,
     T* __restrict__ sim_dst, int line, int j, int L, int NS, int twoff,
     bool first, bool last, int line_words, long long b, long long jline) {
@@ -1326,9 +1326,9 @@ __device__ __forceinline__ void generic_butterfly(
       cplx_t<T> v;
       if (cols) {
         const long long S = a.total / L;
-        v = ld_global<T>(a.in + b * a.in_dist + jline + (long long)idx * S);
+        v = ld_global<T>(in + b * a.in_dist + jline + (long long)idx * S);
       } else {
-        v = ld_global<T>(a.in + b * a.in_dist + idx);
+        v = ld_global<T>(in + b * a.in_dist + idx);
       }
       vr[r] = v.x;
       vi[r] = v.y * a.sign_in;
@@ -1384,13 +1384,13 @@ __device__ __forceinline__ void generic_butterfly(
 // per SM.
 template <typename T, bool WIDE, int BANK>
 __device__ __forceinline__ void generic_dispatch(
-    int R, const GenericArgs<T>& a, const T* sre_src, const T* sim_src,
+    int R, const GenericArgs<T>& a, const cplx_t<T>* in, const T* sre_src, const T* sim_src,
     T* sre_dst, T* sim_dst, int line, int j, int L, int NS, int twoff,
     bool first, bool last, int line_words, long long b, long long jline) {
 #define MOFFT_GENERIC_CASE(RR)                                                  \
   case RR:                                                                      \
-    generic_butterfly<T, RR, BANK>(a, sre_src, sim_src, sre_dst, sim_dst, line, j, L, \
-                             NS, twoff, first, last, line_words, b, jline);     \
+    generic_butterfly<T, RR, BANK>(a, in, sre_src, sim_src, sre_dst, sim_dst, line, j, \
+                             L, NS, twoff, first, last, line_words, b, jline);  \
     break;
   switch (R) {
     MOFFT_GENERIC_CASE(2) MOFFT_GENERIC_CASE(3) MOFFT_GENERIC_CASE(4)
@@ -1401,10 +1401,10 @@ __device__ __forceinline__ void generic_dispatch(
     default:
       if (WIDE) {
         if (R == 32)
-          generic_butterfly<T, 32, BANK>(a, sre_src, sim_src, sre_dst, sim_dst, line, j, L,
+          generic_butterfly<T, 32, BANK>(a, in, sre_src, sim_src, sre_dst, sim_dst, line, j, L,
                                    NS, twoff, first, last, line_words, b, jline);
         else if (R == 64)
-          generic_butterfly<T, 64, BANK>(a, sre_src, sim_src, sre_dst, sim_dst, line, j, L,
+          generic_butterfly<T, 64, BANK>(a, in, sre_src, sim_src, sre_dst, sim_dst, line, j, L,
                                    NS, twoff, first, last, line_words, b, jline);
       }
       break;
@@ -1415,10 +1415,13 @@ __device__ __forceinline__ void generic_dispatch(
 // BANK: the kernel bank whose codelets the stages run (0 default, 1-3 the
 // rewrite families of BankDft).
 template <typename T, bool WIDE, int BANK>
-__global__ void __launch_bounds__(256, WIDE ? 1 : 2) generic_kernel(const GenericArgs<T> args) {
+__global__ void __launch_bounds__(256, WIDE ? 1 : 2)
+generic_kernel(const __grid_constant__ GenericArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  GenericArgs<T> a = args;
-  a.in = after_previous(args.in);
+  // not into a copy of the arguments: the stage loop indexes their radix list,
+  // which would put the copy into local memory (FP32 12870 1.2, FP64 6825 1.3
+  // times the time)
+  const cplx_t<T>* in = after_previous(a.in);
   const int L = a.length;
   const bool cols = a.cols != 0;
   const int line_words = cols ? 0 : spad_len<T>(L);
@@ -1459,8 +1462,8 @@ __global__ void __launch_bounds__(256, WIDE ? 1 : 2) generic_kernel(const Generi
       const long long bb = cols ? b : b + line;
       if (bb >= a.batch) continue;
       const long long jline = cols ? jfirst + line : 0;
-      generic_dispatch<T, WIDE, BANK>(R, a, bufs[cur][0], bufs[cur][1], bufs[cur ^ 1][0],
-                          bufs[cur ^ 1][1], line, j, L, NS, twoff, first, last,
+      generic_dispatch<T, WIDE, BANK>(R, a, in, bufs[cur][0], bufs[cur][1],
+                          bufs[cur ^ 1][0], bufs[cur ^ 1][1], line, j, L, NS, twoff, first, last,
                           line_words, cols ? b : bb, jline);
     }
     __syncthreads();
